@@ -22,11 +22,17 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libtdda.so")
 
-UNITS = ["tdda_kernels.cu", "tdda_api.cu", "tdda_pass_generic.cu", "tdda_pass_z.cu", "tdda_pass_xy.cu",
-         "tdda_pass_zy.cu", "tdda_server.cu", "tdda_pass_xy2.cu", "tdda_pass_dd.cu", "tdda_pass_dd_128.cu", "tdda_pass_dd_192.cu",
-         "tdda_pass_dd_160.cu", "tdda_pass_dd_40.cu"]
+# a unit is a source, or (source, macro, value) compiled once per value; the
+# slowest first, so that the last ones to finish are small
+XY_AXES = (256, 224, 192, 160, 128, 112, 96, 80, 64, 56, 48, 40, 32, 25, 24, 21, 20, 18, 15, 14, 12)
+PLANE_Y = (256, 224, 192, 160, 128, 112, 96, 80, 64, 56, 48, 40, 32)
+UNITS = ([("tdda_axes_xy.cu", "TDDA_AXIS", m) for m in XY_AXES[:5]] +
+         ["tdda_pass_xy2.cu", "tdda_pass_xy.cu", "tdda_pass_zy.cu", "tdda_pass_z.cu", "tdda_axes.cu", "tdda_pass_generic.cu"] +
+         [("tdda_axes_plane.cu", "TDDA_PLANE_MY", m) for m in PLANE_Y] +
+         [("tdda_axes_xy.cu", "TDDA_AXIS", m) for m in XY_AXES[5:]] +
+         ["tdda_kernels.cu", "tdda_api.cu", "tdda_server.cu"])
 HEADERS = ["tdda_fft.cuh", "tdda_fft_ct.cuh", "tdda_internal.cuh", "tdda_device.cuh", "tdda_passes.cuh",
-           "tdda_tensor.cuh", "tdda_session.h"]
+           "tdda_axes.cuh", "tdda_tensor.cuh", "tdda_session.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -54,12 +60,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     jobs = []
     objs = []
     for u in UNITS:
-        src = os.path.join(CSRC, u)
-        obj = os.path.join(BUILD, u + ".o")
+        name, macro, value = u if isinstance(u, tuple) else (u, None, None)
+        src = os.path.join(CSRC, name)
+        obj = os.path.join(BUILD, (name if macro is None else f"{name[:-3]}_{value}.cu") + ".o")
         objs.append(obj)
         if force or _newer(obj, [src] + hdrs):
-            jobs.append([nv] + flags + ["-c", src, "-o", obj])
-    with cf.ThreadPoolExecutor(max_workers=len(UNITS)) as ex:
+            jobs.append([nv] + flags + ([] if macro is None else [f"-D{macro}={value}"]) + ["-c", src, "-o", obj])
+    with cf.ThreadPoolExecutor(max_workers=max(4, min(len(UNITS), os.cpu_count() or 4))) as ex:
         for cmd, res in zip(jobs, ex.map(lambda c: subprocess.run(c, capture_output=True, text=True), jobs)):
             if verbose or res.returncode:
                 sys.stderr.write(res.stdout + res.stderr)

@@ -499,8 +499,35 @@ template <> struct Prec<float> {
     static cudaGraphExec_t& graph(tdda_core* c, int n) { return c->g32.iter[n]; }
 };
 
-// kernels of one A-product at precision T: 3 with the fused z+y passes, else 5
-template <typename T> int product_kernels(const tdda_core* c) { return tdda::zy_fused(c->g, sizeof(T) == 4) ? 3 : 5; }
+// kernels of one A-product at precision T: 3 in the fused forms, else 5
+int product_kernels(const Geom& g, bool fp32) {
+    const tdda::ProductForm f = tdda::product_form(g, fp32);
+    return f == tdda::FORM_FUSED_ZY || f == tdda::FORM_PLANE ? 3 : 5;
+}
+template <typename T> int product_kernels(const tdda_core* c) { return product_kernels(c->g, sizeof(T) == 4); }
+
+// strides and work-grid extents of a geometry whose plans and box are set
+void grid_layout(Geom* g) {
+    g->Hx = g->px.M / 2 + 1;
+    g->Hy = g->py.M / 2 + 1;
+    g->Hz = g->pz.M / 2 + 1;
+    g->sy = g->pz.M;
+    g->sx = (long long)g->py.M * g->pz.M;
+    g->sc = (long long)g->Nx * g->sx;
+    g->sb = 3 * g->sc;
+    const long long Hx = g->Hx, Hy = g->Hy, Hz = g->Hz;
+    if (tdda::axes_lengths(*g)) {  // product threads walk ky
+        g->vb = 3LL * g->px.M * g->py.M * g->Nz;
+        g->gs32 = {3 * Hy * Hz, 1, Hy, Hy * Hz};
+        g->gs64 = {6 * Hy * Hz, 1, Hy, Hy * Hz};
+    } else {  // product threads walk z
+        g->vb = 0;
+        g->gs32 = {3 * Hz, 3 * Hz * Hx, 1, Hz};
+        g->gs64 = {6 * Hz, 6 * Hz * Hx, 6, 1};
+    }
+}
+// entries of the work grid of one right-hand side, whichever form runs
+long long grid_entries(const Geom& g) { return std::max(g.sb, g.vb); }
 
 // right-hand sides per launch of a batch of n: the core's FP32 batch schedule
 template <typename T> int group_size(const tdda_core* c, int n) {
@@ -1052,13 +1079,7 @@ bool shape_geom(const int grid[3], Geom* g) {
     g->Ny = cap_of(grid[1]);
     g->Nz = cap_of(grid[2]);
     g->N = g->Nx * g->Ny * g->Nz;
-    g->Hx = g->px.M / 2 + 1;
-    g->Hy = g->py.M / 2 + 1;
-    g->Hz = g->pz.M / 2 + 1;
-    g->sy = g->pz.M;
-    g->sx = (long long)g->py.M * g->pz.M;
-    g->sc = (long long)g->Nx * g->sx;
-    g->sb = 3 * g->sc;
+    grid_layout(g);
     g->dense = 0;
     g->multi = 1;
     return true;
@@ -1143,7 +1164,8 @@ double core_bytes(int Nx, int Ny, int Nz, int N, int max_rhs) {
     const double Mx = fft_length(Nx, false), My = fft_length(Ny, false), Mz = fft_length(Nz, true);
     const double H = (Mx / 2 + 1) * (My / 2 + 1) * (Mz / 2 + 1);
     const double n3 = 3.0 * N;
-    const double grid = 3.0 * Nx * My * Mz * max_rhs;  // FFT work grid entries
+    // FFT work grid entries: x kept to the lattice, or z (the x-first product)
+    const double grid = 3.0 * My * std::max((double)Nx * Mz, Mx * Nz) * max_rhs;
     return (double)Nx * Ny * Nz * 4 + n3 * 4           // cellmap, R
            + 6 * H * (16 + 8 + 16)                     // Green spectra (FP64, FP32, double-float)
            + grid * (16 + 8)                           // FP64 and FP32 grids
@@ -1164,7 +1186,7 @@ double shape_bytes(const int grid[3], int cap) {
     Geom g;
     if (!shape_geom(grid, &g)) return 0.0;
     const double blk = tdda::max_blocks_per_rhs(g);
-    return (double)g.sb * cap * 8 + cap * (tdda::kPartSlots * blk * 8 + 2 * sizeof(SolveState) +
+    return (double)grid_entries(g) * cap * 8 + cap * (tdda::kPartSlots * blk * 8 + 2 * sizeof(SolveState) +
                                            2 * sizeof(RhsVecs<float>) + tdda::kCounters * 4) +
            8.0 * (grid[0] + grid[1] + grid[2]) + 1e5;
 }
@@ -1220,7 +1242,7 @@ tdda_status shape_create(int device, const int grid[3], int cap, Shape** out) {
         if (cudaDeviceGetAttribute(&c->g.sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) c->g.sms = 0;
     }
     for (int a = 0; a < 3; a++) TDDA_SHAPE_TRY(dalloc_c(c, &c->tw32[a], (size_t)grid[a]));
-    TDDA_SHAPE_TRY(dalloc_c(c, &c->grid32, (size_t)(g.sb * cap)));
+    TDDA_SHAPE_TRY(dalloc_c(c, &c->grid32, (size_t)(grid_entries(g) * cap)));
     TDDA_SHAPE_TRY(dalloc_c(c, &c->rhs32, (size_t)cap + 1));
     TDDA_SHAPE_TRY(dalloc_c(c, &s->rhs32c, (size_t)cap));
     TDDA_SHAPE_TRY(dalloc_c(c, &c->st32, (size_t)cap));
@@ -1587,13 +1609,7 @@ tdda_status core_create(const tdda_core_desc* desc, const tdda::PeriodicImages* 
             return TDDA_ERR_UNSUPPORTED;
         }
     }
-    g.Hx = g.px.M / 2 + 1;
-    g.Hy = g.py.M / 2 + 1;
-    g.Hz = g.pz.M / 2 + 1;
-    g.sy = g.pz.M;
-    g.sx = (long long)g.py.M * g.pz.M;
-    g.sc = (long long)g.Nx * g.sx;
-    g.sb = 3 * g.sc;
+    grid_layout(&g);
     if (tdda::max_pass_smem(g) > tdda::kMaxPassSmem) {
         set_err("FFT grid %dx%dx%d needs more shared memory per tile than a block has", g.px.M, g.py.M, g.pz.M);
         delete c;
@@ -1640,8 +1656,8 @@ tdda_status core_create(const tdda_core_desc* desc, const tdda::PeriodicImages* 
         TDDA_CORE_TRY(dalloc_c(c, &c->tw64[a], (size_t)plans[a]->M));
         TDDA_CORE_TRY(dalloc_c(c, &c->tw32[a], (size_t)plans[a]->M));
     }
-    TDDA_CORE_TRY(dalloc_c(c, &c->grid64, (size_t)(g.sb * c->max_rhs)));
-    TDDA_CORE_TRY(dalloc_c(c, &c->grid32, (size_t)(g.sb * c->max_rhs)));
+    TDDA_CORE_TRY(dalloc_c(c, &c->grid64, (size_t)(grid_entries(g) * c->max_rhs)));
+    TDDA_CORE_TRY(dalloc_c(c, &c->grid32, (size_t)(grid_entries(g) * c->max_rhs)));
     TDDA_CORE_TRY(dalloc_c(c, &c->vin64, n3));
     TDDA_CORE_TRY(dalloc_c(c, &c->vout64, n3));
     TDDA_CORE_TRY(dalloc_c(c, &c->vin32, n3));
@@ -2263,7 +2279,14 @@ unsigned long long tdda_kernel_launches(void) { return g_launches.load(); }
 const char* tdda_core_pass_name(const tdda_core* c, int precision, int pass) {
     if (!c || pass < 0 || pass > 4 || (precision != TDDA_FP64 && precision != TDDA_FP32_REFINE)) return nullptr;
     const bool fp32 = precision == TDDA_FP32_REFINE;
-    const bool fused = tdda::zy_fused(c->g, fp32);
+    const tdda::ProductForm form = tdda::product_form(c->g, fp32);
+    if (form >= tdda::FORM_AXES) {
+        const bool plane = form == tdda::FORM_PLANE;
+        const char* names[5] = {"k_xfwd", plane ? "" : "k_yaxis", plane ? "k_xpass2" : "k_zprod",
+                                plane ? "k_xinv" : "k_yaxis", plane ? "" : "k_xinv"};
+        return names[pass];
+    }
+    const bool fused = form == tdda::FORM_FUSED_ZY;
     switch (pass) {
         case 0: return fused ? "k_zyfwd" : "k_zfwd";
         case 1: return fused ? "" : "k_ypass";
@@ -2275,7 +2298,7 @@ const char* tdda_core_pass_name(const tdda_core* c, int precision, int pass) {
 
 int tdda_core_pass_count(const tdda_core* c, int precision) {
     if (!c || (precision != TDDA_FP64 && precision != TDDA_FP32_REFINE)) return -1;
-    return tdda::zy_fused(c->g, precision == TDDA_FP32_REFINE) ? 3 : 5;
+    return product_kernels(c->g, precision == TDDA_FP32_REFINE);
 }
 
 namespace {
@@ -2460,12 +2483,14 @@ tdda_status tdda_aproduct_noalloc(tdda_core* c, const double* b, double* y) {
     TDDA_TRY(set_device(c->device));
     NoAllocSlot slot;
     TDDA_TRY(noalloc_setup(c->device, &slot));
+    Geom g = c->g;  // the z-y-x passes where the x-first product's grid does not fit
+    g.passes = grid_entries(g) > (long long)kNoAllocGridElems;
     RhsVecs<double> v{};
     v.p = (double2*)b;
     v.Ap = (double2*)y;
     TDDA_CK(cudaMemcpyAsync(slot.rhs, &v, sizeof(v), cudaMemcpyHostToDevice, c->stream));
     count_launches(5);
-    TDDA_CK(tdda::launch_aproduct<double>(c->g, tdda::SRC_IN, tdda::SNK_OUT, 1, slot.rhs, c->green64, c->tw64[0],
+    TDDA_CK(tdda::launch_aproduct<double>(g, tdda::SRC_IN, tdda::SNK_OUT, 1, slot.rhs, c->green64, c->tw64[0],
                                           c->tw64[1], c->tw64[2], c->cellmap, slot.grid, c->stream));
     TDDA_CK(cudaStreamSynchronize(c->stream));
     return TDDA_OK;

@@ -77,24 +77,29 @@ __device__ __forceinline__ bool finite2(double2 a) { return isfinite(a.x) && isf
 template <typename T> __device__ __forceinline__ cx<T> from_d(double2 a) { return mk<T>(T(a.x), T(a.y)); }
 
 // ------------------------------------------------------------ reductions
-// Block-wide sum of NV doubles in a fixed order; the result is valid in
+// Block-wide sum of NV doubles in a fixed order; the results are valid in
 // thread 0.  sred must hold NV * blockDim.x doubles.  The partials go through
-// shared memory and one warp adds them: on GB300 every FP64 warp instruction
-// occupies the narrow FP64 pipe for many cycles, so one warp summing the block
-// costs far less than a shuffle tree run by every warp.
+// shared memory and one warp adds each value (warp k value k, where there are
+// that many): on GB300 every FP64 warp instruction occupies its SM quarter's
+// narrow FP64 pipe for 64 cycles, so a shuffle tree in every warp would cost
+// far more, and one warp adding all values took NV times as long.
 template <int NV> __device__ __forceinline__ void block_sum(double (&v)[NV], double* sred) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = blockDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = blockDim.x, nw = nt >> 5;
 #pragma unroll
     for (int k = 0; k < NV; k++) sred[k * nt + threadIdx.x] = v[k];
     __syncthreads();
-    if (warp == 0) {
 #pragma unroll
-        for (int k = 0; k < NV; k++) {
-            double a = 0.0;
-            for (int i = lane; i < nt; i += 32) a += sred[k * nt + i];
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-            v[k] = a;
-        }
+    for (int k = 0; k < NV; k++) {
+        if (k % nw != warp) continue;
+        double a = 0.0;
+        for (int i = lane; i < nt; i += 32) a += sred[k * nt + i];
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        if (lane == 0) sred[k * nt] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = sred[k * nt];
     }
     __syncthreads();
 }
@@ -223,9 +228,9 @@ template <typename T> using tot_t = typename std::conditional<sizeof(T) == 4, fl
 // Shared scratch of a reduction kernel, in doubles: NV * nt for the FP64
 // block sum, 32 * NV float2 (8 bytes each, one per warp slot) for the
 // double-float one.
-template <typename T, int NV> __host__ __device__ constexpr int sred_size() {
+template <typename T, int NV> __host__ __device__ constexpr int sred_size(int nt = kNT) {
     static_assert(sizeof(float2) == sizeof(double), "a float2 slot is one double");
-    return sizeof(T) == 4 ? 32 * NV : NV * kNT;
+    return sizeof(T) == 4 ? 32 * NV : NV * nt;
 }
 
 // The end of one BiCGSTAB step, given r0.r and |r|^2 of the new residual
@@ -373,7 +378,7 @@ __device__ __forceinline__ StepIn load_step_in(const SolveState* st, int p) {
 
 // The end of step k - 1 as seen by step k (parity p): zeta = At.t / At.At in
 // FP32; r0.r and |r|^2 of r = t - zeta At as FP64 multiply-adds on the
-// double-float totals (they cancel as r gets small next to t); then the
+// double-float sums (they cancel as r gets small next to t); then the
 // logic of DDAModel.cpp:218-255: convergence (not after the initial
 // products), the iteration limit, breakdown on r0.rl = 0, beta.
 struct StepEnd {
@@ -381,17 +386,35 @@ struct StepEnd {
     float err;
     int it, stop, set_iterations, iterations;
 };
-__device__ __forceinline__ double df_d(float2 a) { return (double)a.x + (double)a.y; }
-__device__ __forceinline__ StepEnd step_end_f32(const StepIn& st, const float2 (&tot)[8]) {
+// Run by one full warp, the totals (8) in shared memory and st in lane 0; the
+// result is lane 0's.  An FP64 instruction holds its SM quarter's pipe for 64
+// cycles whatever its active lanes, and this is a serial chain every block of a
+// gather waits for: the eight totals become FP64 in eight lanes at once, and
+// the three sums (real and imaginary part of r0.r, |r|^2) run as one
+// instruction sequence in three lanes -- 12 FP64 instructions instead of 40.
+__device__ __forceinline__ StepEnd step_end_f32(const StepIn& st, const float2* tot) {
     StepEnd e;
+    const int lane = threadIdx.x & 31;
     e.zeta = fdiv2(make_float2(tot[0].x, tot[1].x), make_float2(tot[2].x, 0.f));  // DDAModel.cpp:225
     const double zx = e.zeta.x, zy = e.zeta.y;
-    const double ax = df_d(tot[0]), ay = df_d(tot[1]), bb = df_d(tot[2]);
-    const double tx = df_d(tot[3]), ty = df_d(tot[4]), ux = df_d(tot[5]), uy = df_d(tot[6]), cc = df_d(tot[7]);
-    e.rho = make_float2((float)(tx - (zx * ux - zy * uy)), (float)(ty - (zx * uy + zy * ux)));
-    double rn2 = cc - 2.0 * (zx * ax + zy * ay) + (zx * zx + zy * zy) * bb;
-    if (!(rn2 > 0.0)) rn2 = isnan(rn2) ? rn2 : 0.0;
-    e.err = sqrtf((float)rn2) / st.Enorm;
+    const float2 mine = tot[lane & 7];
+    const double d = (double)mine.x + (double)mine.y;
+    // lane 0: r0.t.x - (zx ux - zy uy); lane 1: r0.t.y - (zx uy + zy ux), u = r0.At;
+    // lane 2: t.t - 2 (zx ax + zy ay) + |zeta|^2 At.At, a = At.t
+    const double c0 = __shfl_sync(0xffffffffu, d, lane == 0 ? 3 : lane == 1 ? 4 : 7);
+    const double c1 = __shfl_sync(0xffffffffu, d, lane == 0 ? 5 : lane == 1 ? 6 : 0);
+    const double c2 = __shfl_sync(0xffffffffu, d, lane == 0 ? 6 : lane == 1 ? 5 : 1);
+    const double bb = __shfl_sync(0xffffffffu, d, 2);
+    const double zs = lane == 0 ? -zy : zy;
+    double v = fma(lane == 2 ? -2.0 : -1.0, fma(zx, c1, zs * c2), c0);
+    const double q = fma(fma(zx, zx, zy * zy), bb, v);
+    if (lane == 2) {
+        v = q;
+        if (!(v > 0.0)) v = isnan(v) ? v : 0.0;
+    }
+    const float f = (float)v;
+    e.rho = make_float2(__shfl_sync(0xffffffffu, f, 0), __shfl_sync(0xffffffffu, f, 1));
+    e.err = sqrtf(__shfl_sync(0xffffffffu, f, 2)) / st.Enorm;
     const bool init = st.init != 0;
     e.it = st.it + (init ? 0 : 1);
     e.stop = ST_RUNNING;

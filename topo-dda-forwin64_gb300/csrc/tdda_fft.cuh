@@ -115,6 +115,8 @@ template <typename T> __device__ __forceinline__ cx<T> bsub(cx<T> a, cx<T> b) { 
 template <typename T> __device__ __forceinline__ cx<T> bfma(cx<T> a, T c, cx<T> acc) {
     return mk<T>(acc.x + c * a.x, acc.y + c * a.y);
 }
+// c a for a real constant c
+template <typename T> __device__ __forceinline__ cx<T> bscale(cx<T> a, T c) { return cscale<T>(a, c); }
 template <> __device__ __forceinline__ float2 badd<float>(float2 a, float2 b) {
     unsigned long long r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(b)));
@@ -129,6 +131,11 @@ template <> __device__ __forceinline__ float2 bfma<float>(float2 a, float c, flo
     unsigned long long r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(make_float2(c, c))),
         "l"(f2_pack(acc)));
+    return f2_unpack(r);
+}
+template <> __device__ __forceinline__ float2 bscale<float>(float2 a, float c) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_pack(a)), "l"(f2_pack(make_float2(c, c))));
     return f2_unpack(r);
 }
 
@@ -183,9 +190,9 @@ template <int SIGN, typename T> struct Bfly<4, SIGN, T> {
 };
 
 // DFT of length R whose inputs v[NIN .. R) are zero: they are neither read
-// nor added (the zero-padded half of a first stage).  Pruned forms for NIN =
-// R / 2 with R = 4, 8, 16 (the first radices of the two-stage plans); any
-// other NIN runs the full butterfly on zeros.
+// nor added (the zero-padded half of a first stage).  Pruned forms for radix 4
+// and 8 with half their inputs, and for the odd and composite radices below;
+// any other NIN runs the full butterfly on zeros.
 template <int R, int SIGN, typename T, int NIN> struct BflyIn {
     static __device__ __forceinline__ void run(cx<T>* v) {
 #pragma unroll
@@ -218,17 +225,25 @@ template <int SIGN, typename T, int NIN4> struct Bfly8 {
         BflyIn<4, SIGN, T, NIN4>::run(e);
         BflyIn<4, SIGN, T, NIN4>::run(o);
         // W8^1 = (1 + SIGN i) sqrt(1/2), W8^2 = SIGN i, W8^3 = (-1 + SIGN i) sqrt(1/2)
-        cx<T> o1 = mk<T>((o[1].x - T(SIGN) * o[1].y) * h, (o[1].y + T(SIGN) * o[1].x) * h);
-        cx<T> o2 = cmul_i<SIGN, T>(o[2]);
-        cx<T> o3 = mk<T>((-o[3].x - T(SIGN) * o[3].y) * h, (-o[3].y + T(SIGN) * o[3].x) * h);
+        const cx<T> t1 = mk<T>(o[1].x - T(SIGN) * o[1].y, o[1].y + T(SIGN) * o[1].x);
+        const cx<T> t3 = mk<T>(-o[3].x - T(SIGN) * o[3].y, -o[3].y + T(SIGN) * o[3].x);
+        const cx<T> o2 = cmul_i<SIGN, T>(o[2]);
         v[0] = badd<T>(e[0], o[0]);
         v[4] = bsub<T>(e[0], o[0]);
-        v[1] = badd<T>(e[1], o1);
-        v[5] = bsub<T>(e[1], o1);
         v[2] = badd<T>(e[2], o2);
         v[6] = bsub<T>(e[2], o2);
-        v[3] = badd<T>(e[3], o3);
-        v[7] = bsub<T>(e[3], o3);
+        if constexpr (is_dd<T>) {  // a double-float product costs more than the sum it would save
+            const cx<T> o1 = cscale<T>(t1, h), o3 = cscale<T>(t3, h);
+            v[1] = badd<T>(e[1], o1);
+            v[5] = bsub<T>(e[1], o1);
+            v[3] = badd<T>(e[3], o3);
+            v[7] = bsub<T>(e[3], o3);
+        } else {  // e +/- sqrt(1/2) t as one fused multiply-add each
+            v[1] = bfma<T>(t1, h, e[1]);
+            v[5] = bfma<T>(t1, -h, e[1]);
+            v[3] = bfma<T>(t3, h, e[3]);
+            v[7] = bfma<T>(t3, -h, e[3]);
+        }
     }
 };
 template <int SIGN, typename T> struct Bfly<8, SIGN, T> : Bfly8<SIGN, T, 4> {};
@@ -269,19 +284,22 @@ template <> struct OddConst<7> {
     }
 };
 
-template <int R, int SIGN, typename T> struct BflyOdd {
+// NIN < R: the inputs v[NIN .. R) are zero.
+template <int R, int SIGN, typename T, int NIN = R> struct BflyOdd {
     static __device__ __forceinline__ void run(cx<T>* v) {
         constexpr int H = (R - 1) / 2;
-        cx<T> sp[H], sm[H];
+        static_assert(NIN >= 1 && NIN <= R, "inputs of an odd butterfly");
+        cx<T> sp[H], sm[H];  // pairs (r, R - r): sum and difference, v[r] itself where v[R - r] is zero
 #pragma unroll
         for (int r = 1; r <= H; r++) {
-            sp[r - 1] = badd<T>(v[r], v[R - r]);
-            sm[r - 1] = bsub<T>(v[r], v[R - r]);
+            sp[r - 1] = R - r < NIN ? badd<T>(v[r], v[R - r]) : v[r];
+            sm[r - 1] = R - r < NIN ? bsub<T>(v[r], v[R - r]) : v[r];
         }
         cx<T> out[R];
         cx<T> s0 = v[0];
 #pragma unroll
-        for (int r = 0; r < H; r++) s0 = badd<T>(s0, sp[r]);
+        for (int r = 0; r < H; r++)
+            if (r + 1 < NIN) s0 = badd<T>(s0, sp[r]);
         out[0] = s0;
 #pragma unroll
         for (int q = 1; q <= H; q++) {
@@ -289,10 +307,11 @@ template <int R, int SIGN, typename T> struct BflyOdd {
             cx<T> im = czero<T>();
 #pragma unroll
             for (int r = 1; r <= H; r++) {
+                if (r >= NIN) continue;
                 const T c = T(OddConst<R>::c(r * q));
                 const T s = T(OddConst<R>::s(r * q));
                 re = bfma<T>(sp[r - 1], c, re);
-                im = bfma<T>(sm[r - 1], s, im);
+                im = r == 1 ? bscale<T>(sm[0], s) : bfma<T>(sm[r - 1], s, im);
             }
             cx<T> rot = cmul_i<SIGN, T>(im);  // SIGN i * im
             out[q] = badd<T>(re, rot);
@@ -305,6 +324,12 @@ template <int R, int SIGN, typename T> struct BflyOdd {
 template <int SIGN, typename T> struct Bfly<3, SIGN, T> : BflyOdd<3, SIGN, T> {};
 template <int SIGN, typename T> struct Bfly<5, SIGN, T> : BflyOdd<5, SIGN, T> {};
 template <int SIGN, typename T> struct Bfly<7, SIGN, T> : BflyOdd<7, SIGN, T> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<3, SIGN, T, NIN> : BflyOdd<3, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<5, SIGN, T, NIN> : BflyOdd<5, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<7, SIGN, T, NIN> : BflyOdd<7, SIGN, T, NIN> {};
+template <int SIGN, typename T> struct BflyIn<2, SIGN, T, 1> {
+    static __device__ __forceinline__ void run(cx<T>* v) { v[1] = v[0]; }
+};
 
 // ------------------------------------------------------ composite butterflies
 // DFT of length R = R1 R2 in registers: with n = R2 n1 + n2 and k = k1 + R1 k2,
@@ -312,6 +337,16 @@ template <int SIGN, typename T> struct Bfly<7, SIGN, T> : BflyOdd<7, SIGN, T> {}
 // R2 DFTs of length R1, twiddles W_R^(n2 k1), R1 DFTs of length R2.  The
 // constants cos / sin(2 pi m / R) are tabulated below.
 template <int R> struct RootTab;
+template <> struct RootTab<6> {
+    static __device__ __forceinline__ double c(int m) {
+        constexpr double t[6] = {1.0, 0.5, -0.5, -1.0, -0.5, 0.5};
+        return t[m % 6];
+    }
+    static __device__ __forceinline__ double s(int m) {
+        constexpr double t[6] = {0.0, 0.8660254037844386, 0.8660254037844387, 0.0, -0.8660254037844384, -0.8660254037844386};
+        return t[m % 6];
+    }
+};
 template <> struct RootTab<10> {
     static __device__ __forceinline__ double c(int m) {
         constexpr double t[10] = {1, 0.80901699437494745, 0.30901699437494745, -0.30901699437494734, -0.80901699437494734, -1, -0.80901699437494756, -0.30901699437494756, 0.30901699437494723, 0.80901699437494734};
@@ -330,6 +365,16 @@ template <> struct RootTab<12> {
     static __device__ __forceinline__ double s(int m) {
         constexpr double t[12] = {0, 0.49999999999999994, 0.8660254037844386, 1, 0.86602540378443871, 0.49999999999999994, 1.2246467991473532e-16, -0.49999999999999972, -0.86602540378443837, -1, -0.8660254037844386, -0.50000000000000044};
         return t[m % 12];
+    }
+};
+template <> struct RootTab<14> {
+    static __device__ __forceinline__ double c(int m) {
+        constexpr double t[14] = {1.0, 0.9009688679024191, 0.6234898018587336, 0.22252093395631445, -0.22252093395631434, -0.6234898018587335, -0.900968867902419, -1.0, -0.9009688679024191, -0.6234898018587337, -0.2225209339563146, 0.22252093395631334, 0.6234898018587334, 0.9009688679024194};
+        return t[m % 14];
+    }
+    static __device__ __forceinline__ double s(int m) {
+        constexpr double t[14] = {0.0, 0.4338837391175581, 0.7818314824680298, 0.9749279121818236, 0.9749279121818236, 0.7818314824680299, 0.43388373911755823, 0.0, -0.433883739117558, -0.7818314824680297, -0.9749279121818236, -0.9749279121818238, -0.7818314824680299, -0.4338837391175575};
+        return t[m % 14];
     }
 };
 template <> struct RootTab<16> {
@@ -354,27 +399,64 @@ template <> struct RootTab<24> {
     }
 };
 
-// NIN1 < R1: only inputs n1 < NIN1 of each inner DFT (v[0 .. R2 NIN1)) are
-// non-zero.
-template <int R1, int R2, int SIGN, typename T, int NIN1 = R1> struct BflyComp {
-    static __device__ __forceinline__ void run(cx<T>* v) {
-        constexpr int R = R1 * R2;
-        cx<T> y[R2][R1];
-#pragma unroll
-        for (int n2 = 0; n2 < R2; n2++) {
+template <> struct RootTab<20> {
+    static __device__ __forceinline__ double c(int m) {
+        constexpr double t[20] = {1.0, 0.9510565162951535, 0.8090169943749475, 0.5877852522924731, 0.30901699437494745, 0.0, -0.30901699437494734, -0.587785252292473, -0.8090169943749473, -0.9510565162951535, -1.0, -0.9510565162951538, -0.8090169943749476, -0.5877852522924732, -0.30901699437494756, 0.0, 0.30901699437494723, 0.5877852522924729, 0.8090169943749473, 0.9510565162951535};
+        return t[m % 20];
+    }
+    static __device__ __forceinline__ double s(int m) {
+        constexpr double t[20] = {0.0, 0.3090169943749474, 0.5877852522924731, 0.8090169943749475, 0.9510565162951535, 1.0, 0.9510565162951536, 0.8090169943749475, 0.5877852522924732, 0.3090169943749475, 0.0, -0.3090169943749469, -0.587785252292473, -0.8090169943749473, -0.9510565162951535, -1.0, -0.9510565162951536, -0.8090169943749476, -0.5877852522924734, -0.3090169943749476};
+        return t[m % 20];
+    }
+};
+template <> struct RootTab<28> {
+    static __device__ __forceinline__ double c(int m) {
+        constexpr double t[28] = {1.0, 0.9749279121818236, 0.9009688679024191, 0.7818314824680298, 0.6234898018587336, 0.4338837391175582, 0.22252093395631445, 0.0, -0.22252093395631434, -0.43388373911755806, -0.6234898018587335, -0.7818314824680295, -0.900968867902419, -0.9749279121818237, -1.0, -0.9749279121818237, -0.9009688679024191, -0.7818314824680296, -0.6234898018587337, -0.4338837391175583, -0.2225209339563146, 0.0, 0.22252093395631334, 0.43388373911755795, 0.6234898018587334, 0.7818314824680297, 0.9009688679024194, 0.9749279121818235};
+        return t[m % 28];
+    }
+    static __device__ __forceinline__ double s(int m) {
+        constexpr double t[28] = {0.0, 0.2225209339563144, 0.4338837391175581, 0.6234898018587335, 0.7818314824680298, 0.9009688679024191, 0.9749279121818236, 1.0, 0.9749279121818236, 0.9009688679024191, 0.7818314824680299, 0.6234898018587339, 0.43388373911755823, 0.2225209339563141, 0.0, -0.22252093395631384, -0.433883739117558, -0.6234898018587338, -0.7818314824680297, -0.900968867902419, -0.9749279121818236, -1.0, -0.9749279121818238, -0.9009688679024193, -0.7818314824680299, -0.6234898018587337, -0.4338837391175575, -0.22252093395631464};
+        return t[m % 28];
+    }
+};
+template <> struct RootTab<32> {
+    static __device__ __forceinline__ double c(int m) {
+        constexpr double t[32] = {1.0, 0.9807852804032304, 0.9238795325112867, 0.8314696123025452, 0.7071067811865476, 0.5555702330196023, 0.38268343236508984, 0.19509032201612833, 0.0, -0.1950903220161282, -0.3826834323650897, -0.555570233019602, -0.7071067811865475, -0.8314696123025453, -0.9238795325112867, -0.9807852804032304, -1.0, -0.9807852804032304, -0.9238795325112868, -0.8314696123025455, -0.7071067811865477, -0.5555702330196022, -0.38268343236509034, -0.19509032201612866, 0.0, 0.1950903220161283, 0.38268343236509, 0.5555702330196018, 0.7071067811865474, 0.8314696123025452, 0.9238795325112865, 0.9807852804032303};
+        return t[m % 32];
+    }
+    static __device__ __forceinline__ double s(int m) {
+        constexpr double t[32] = {0.0, 0.19509032201612825, 0.3826834323650898, 0.5555702330196022, 0.7071067811865475, 0.8314696123025452, 0.9238795325112867, 0.9807852804032304, 1.0, 0.9807852804032304, 0.9238795325112867, 0.8314696123025455, 0.7071067811865476, 0.5555702330196022, 0.3826834323650899, 0.1950903220161286, 0.0, -0.19509032201612836, -0.38268343236508967, -0.555570233019602, -0.7071067811865475, -0.8314696123025452, -0.9238795325112865, -0.9807852804032303, -1.0, -0.9807852804032304, -0.9238795325112866, -0.8314696123025455, -0.7071067811865477, -0.5555702330196022, -0.3826834323650904, -0.19509032201612872};
+        return t[m % 32];
+    }
+};
+// a times exp(SIGN 2 pi i m / R) for a compile-time m; the quarter turns are exact
+template <int R, int SIGN, typename T> __device__ __forceinline__ cx<T> rotate_root(cx<T> a, int m) {
+    const int k = m % R;
+    if (k == 0) return a;
+    if (4 * k == R) return cmul_i<SIGN, T>(a);
+    if (2 * k == R) return mk<T>(-a.x, -a.y);
+    if (4 * k == 3 * R) return cmul_i<-SIGN, T>(a);
+    const T c = T(RootTab<R>::c(k)), s = T(SIGN) * T(RootTab<R>::s(k));
+    return mk<T>(a.x * c - a.y * s, a.x * s + a.y * c);
+}
+// NIN < R1 R2: the inputs v[NIN .. R1 R2) are zero, so the inner DFT of n2
+// takes only its first ceil((NIN - n2) / R2) inputs.
+template <int R1, int R2, int SIGN, typename T, int NIN = R1 * R2> struct BflyComp {
+    template <int N2> static __device__ __forceinline__ void inner(const cx<T>* v, cx<T> (&y)[R2][R1]) {
+        if constexpr (N2 < R2) {
+            constexpr int n = NIN > N2 ? (NIN - N2 + R2 - 1) / R2 : 1;  // at least one (a zero) for tiny NIN
             cx<T> a[R1];
 #pragma unroll
-            for (int n1 = 0; n1 < NIN1; n1++) a[n1] = v[R2 * n1 + n2];
-            BflyIn<R1, SIGN, T, NIN1>::run(a);
+            for (int n1 = 0; n1 < n; n1++) a[n1] = R2 * n1 + N2 < NIN ? v[R2 * n1 + N2] : czero<T>();
+            BflyIn<R1, SIGN, T, n>::run(a);
 #pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) {
-                if (n2 > 0 && k1 > 0) {
-                    const T c = T(RootTab<R>::c(n2 * k1)), s = T(SIGN) * T(RootTab<R>::s(n2 * k1));
-                    a[k1] = mk<T>(a[k1].x * c - a[k1].y * s, a[k1].x * s + a[k1].y * c);
-                }
-                y[n2][k1] = a[k1];
-            }
+            for (int k1 = 0; k1 < R1; k1++) y[N2][k1] = rotate_root<R1 * R2, SIGN, T>(a[k1], N2 * k1);
+            inner<N2 + 1>(v, y);
         }
+    }
+    static __device__ __forceinline__ void run(cx<T>* v) {
+        cx<T> y[R2][R1];
+        inner<0>(v, y);
 #pragma unroll
         for (int k1 = 0; k1 < R1; k1++) {
             cx<T> b[R2];
@@ -386,14 +468,25 @@ template <int R1, int R2, int SIGN, typename T, int NIN1 = R1> struct BflyComp {
         }
     }
 };
-template <int SIGN, typename T> struct Bfly<16, SIGN, T> : BflyComp<4, 4, SIGN, T> {};
-template <int SIGN, typename T> struct BflyIn<8, SIGN, T, 4> : Bfly8<SIGN, T, 2> {};
-template <int SIGN, typename T> struct BflyIn<16, SIGN, T, 8> : BflyComp<4, 4, SIGN, T, 2> {};
-template <int SIGN, typename T> struct Bfly<24, SIGN, T> : BflyComp<8, 3, SIGN, T> {};
-template <int SIGN, typename T> struct BflyIn<24, SIGN, T, 12> : BflyComp<8, 3, SIGN, T, 4> {};
-template <int SIGN, typename T> struct BflyIn<12, SIGN, T, 6> : BflyComp<4, 3, SIGN, T, 2> {};
-template <int SIGN, typename T> struct Bfly<12, SIGN, T> : BflyComp<4, 3, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<6, SIGN, T> : BflyComp<2, 3, SIGN, T> {};
 template <int SIGN, typename T> struct Bfly<10, SIGN, T> : BflyComp<2, 5, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<12, SIGN, T> : BflyComp<4, 3, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<14, SIGN, T> : BflyComp<2, 7, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<16, SIGN, T> : BflyComp<4, 4, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<24, SIGN, T> : BflyComp<8, 3, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<20, SIGN, T> : BflyComp<4, 5, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<28, SIGN, T> : BflyComp<4, 7, SIGN, T> {};
+template <int SIGN, typename T> struct Bfly<32, SIGN, T> : BflyComp<8, 4, SIGN, T> {};
+template <int SIGN, typename T> struct BflyIn<8, SIGN, T, 4> : Bfly8<SIGN, T, 2> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<6, SIGN, T, NIN> : BflyComp<2, 3, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<10, SIGN, T, NIN> : BflyComp<2, 5, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<12, SIGN, T, NIN> : BflyComp<4, 3, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<14, SIGN, T, NIN> : BflyComp<2, 7, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<16, SIGN, T, NIN> : BflyComp<4, 4, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<20, SIGN, T, NIN> : BflyComp<4, 5, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<24, SIGN, T, NIN> : BflyComp<8, 3, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<28, SIGN, T, NIN> : BflyComp<4, 7, SIGN, T, NIN> {};
+template <int SIGN, typename T, int NIN> struct BflyIn<32, SIGN, T, NIN> : BflyComp<8, 4, SIGN, T, NIN> {};
 
 // ----------------------------------------------------------------- one stage
 // Out-of-place (ping-pong) stage: reads x, writes y, then a barrier.  Each

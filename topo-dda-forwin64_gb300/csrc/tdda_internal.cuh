@@ -3,11 +3,16 @@
 //
 // HBM layout of one core (one lattice at one wavelength):
 //   cellmap   int32 [Nx][Ny][Nz]          dipole index of each cell, -1 if empty
-//   green64   double2 [Hy][Hx][Hz][6]     folded Green spectrum / (Mx My Mz)
-//   green32   float2  [Hy][Hx][3][Hz][2]  the same rounded to FP32 (mixed path), as
+//   green64   double2 [Hx][6][Hz][Hy]     folded Green spectrum / (Mx My Mz)
+//   green32   float2  [Hx][3][Hz][Hy][2]  the same rounded to FP32 (mixed path), as
 //                                         planes of component pairs (xx|xy, xz|yy, yz|zz)
+//             (for the lengths of the x-first product, tdda_axes.cuh, whose product
+//             threads walk ky; [Hy][Hx][Hz][6] and [Hy][Hx][3][Hz][2] for the others,
+//             whose product threads walk z.  Geom::gs32 / gs64 hold the strides)
 //   tw{x,y,z} double2/float2 [M]          exp(-2 pi i m / M)
-//   grid      cx<T> [nrhs][3][Nx][My][Mz]  FFT work grid (x kept to the lattice)
+//   grid      FFT work grid, cx<T> [nrhs][3][Nx][My][Mz] (x kept to the lattice), or in
+//             the x-first product [nrhs][Mx] planes of the lattice's z (FP32
+//             component-major, FP64 component fastest)
 // with H = M/2 + 1 per axis (the tensor components are even or odd in each
 // axis, so the spectrum at M-k equals +/- the spectrum at k).
 #pragma once
@@ -19,19 +24,30 @@
 
 namespace tdda {
 
+// strides of the folded Green spectrum: entries for FP64 and double-float
+// tables (l: component), pairs of components for the FP32 table (l: pair)
+struct GreenStride {
+    long long x, y, z, l;
+};
+
 struct Geom {
     int Nx, Ny, Nz;    // lattice box
     int N;             // dipoles
     AxisPlan px, py, pz;
     int Hx, Hy, Hz;    // folded Green extents
     long long sy, sx, sc, sb;  // grid strides (y, x, component, rhs) in elements
+    long long vb;      // rhs stride of the x-first product's work grid
+    GreenStride gs32, gs64;
+    int passes;        // 1: the z-y-x passes whatever the lengths (a work grid too small
+                       // for the x-first product's)
     int dense;         // 1: the full box in build_a_bulk order, dipole (x Ny + y) Nz + z
                        // in every cell (tools.cpp:497-510), so no cellmap lookup
     // FP32 x pass (set by tdda_core_set_xpass / tdda_core_autotune):
-    int x_form;        // 0: the register form on a two-stage plan where one is compiled,
+    int x_form;        // 0: the x-first product where its lengths are compiled, else the
+                       // register form on a two-stage plan where one is compiled;
                        // 1: the shared-memory form on the length's compiled plan
-    int x_tile;        // z-columns per block of the register form: 8, 16, or 0 for
-                       // the built-in choice (16 for M = 128, else 8)
+    int x_tile;        // lines per block of the x-first gather, or z-columns per block of
+                       // the register form: 8, 16, or 0 for the built-in choice
     int multi;         // 1: a cross-lattice batch -- every right-hand side brings its own
                        // lattice (RhsVecs::Nx ... green); Nx, Ny, Nz, N above are the
                        // largest the grid shape holds (the strides follow them)
@@ -208,13 +224,35 @@ template <typename T> bool pass_ct_xy(int pass, int mode, const PassArgs<T>& a, 
 template <typename T> bool pass_zy(int pass, int mode, const PassArgs<T>& a, cudaError_t* err);
 bool zy_fused(const Geom& g, bool fp32);
 cudaError_t configure_pass_zy();
-// the double-float A-product (tdda_pass_dd.cu): residual r = E - (A P + al P)
+// ------------------------------------------------------------ x-first product
+// tdda_axes.cuh: lengths of the x and y kernels, of the z kernels, and the
+// (y, z) lengths of the fused FP32 plane kernels (those that fit a block)
+#define TDDA_XY_AXES(X)                                                                                       \
+    X(12) X(14) X(15) X(18) X(20) X(21) X(24) X(25) X(32) X(40) X(48) X(56) X(64) X(80) X(96) X(112) X(128) \
+    X(160) X(192) X(224) X(256)
+#define TDDA_Z_AXES(X) X(12) X(14) X(15) X(20) X(21) X(24) X(25) X(32) X(40) X(48) X(56) X(64)
+#define TDDA_PLANE_Y(X) X(32) X(40) X(48) X(56) X(64) X(80) X(96) X(112) X(128) X(160) X(192) X(224) X(256)
+#define TDDA_PLANE_Z(X) X(20) X(24) X(32) X(40) X(48) X(56) X(64)
+enum AxisOp : int { AXIS_XFWD = 0, AXIS_XINV = 1, AXIS_YFWD = 2, AXIS_YINV = 3 };
+// every axis has x-first kernels / the FP32 planes have a fused kernel
+bool axes_lengths(const Geom& g);
+bool axes_plane(const Geom& g);
+int axis_tile_fwd(const Geom& g);  // FP32 lines per block of k_xfwd / k_xinv
+int axis_tile_inv(const Geom& g);
+int axis_sink_blocks(const Geom& g, bool fp32);
+// one x-first product: 5 kernels, or 3 with the fused plane kernel; ev as launch_aproduct
+template <typename T> cudaError_t launch_axes(int src, int snk, const PassArgs<T>& a, bool plane, cudaEvent_t* ev);
+cudaError_t configure_axes();
+// kernels of an A-product (how launch_aproduct runs it)
+enum ProductForm : int { FORM_PASSES = 0, FORM_FUSED_ZY = 1, FORM_AXES = 2, FORM_PLANE = 3 };
+ProductForm product_form(const Geom& g, bool fp32);
+
+// the double-float A-product (x-first): residual r = E - (A P + al P)
 // of the FP64 vectors of rhs (laid out as RhsVecs<double>), for the grids
 // dd_lengths() accepts
 bool dd_lengths(const Geom& g);
 cudaError_t launch_residual_dd(const Geom& g, int nrhs, const RhsVecs<dd>* rhs, const dd2* green, const dd2* twx,
                                const dd2* twy, const dd2* twz, const int* cellmap, dd2* grid, cudaStream_t stream);
-cudaError_t configure_pass_dd();
 // dst = src split into double-float pairs
 cudaError_t launch_to_dd(long long n, const double2* src, dd2* dst, cudaStream_t stream);
 cudaError_t configure_pass_generic();
@@ -253,7 +291,7 @@ cudaError_t launch_sici_table(double* si, double* ci, cudaStream_t stream);
 
 // One A-product over nrhs right-hand sides.  rhs[] lives in device memory.
 // ev, when given, holds 6 events recorded before K1..K5 and after K5; with
-// the fused z+y passes ev[1] = ev[2] and ev[4] = ev[5] (K2 and K4 take no time).
+// the fused forms ev[1] = ev[2] and ev[4] = ev[5] (K2 and K5 take no time).
 // For SRC_IN with SNK_OUT / SNK_ALB the vectors used are rhs[b].p (input)
 // and rhs[b].Ap (output); SNK_RES reads P and E and writes r, r0, p.
 template <typename T>

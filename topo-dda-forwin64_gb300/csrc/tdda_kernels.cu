@@ -31,15 +31,19 @@ namespace {
 
 using namespace dev;
 // ================================================================ K6 update
+// 128 threads: each SM quarter's FP64 pipe serves its own warps, so many small
+// blocks keep every quarter busy (12,000 entries: 24.5 -> 6 us against 4
+// entries a thread in blocks of 256).
+constexpr int kNTUpdate = 128;
 template <typename T>
-__global__ void __launch_bounds__(kNT) k_update(int n3, const RhsVecs<T>* __restrict__ rhs, int is_init) {
+__global__ void __launch_bounds__(kNTUpdate) k_update(int n3, const RhsVecs<T>* __restrict__ rhs, int is_init) {
     static_assert(sizeof(T) == 8, "the FP32 step is the deferred form");
-    __shared__ double sred[sred_size<T, 4>()];
+    __shared__ double sred[sred_size<T, 3>(kNTUpdate)];
     const int b = blockIdx.y;
     const RhsVecs<T> R = rhs[b];
     if (rhs_done(R.st)) return;
     const cx<T> alpha = st_alpha<T>(R.st), zeta = st_zeta<T>(R.st);
-    acc_t<T> acc[4] = {0, 0, 0, 0};
+    acc_t<T> acc[3] = {0, 0, 0};
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n3; e += gridDim.x * blockDim.x) {
         const cx<T> Ap = R.Ap[e], r = R.r[e], p = R.p[e], t = R.t[e], At = R.At[e], r0 = R.r0[e];
         cx<T> P = R.P[e];
@@ -54,8 +58,8 @@ __global__ void __launch_bounds__(kNT) k_update(int n3, const RhsVecs<T>* __rest
         acc[1] += r0.x * rn.y - r0.y * rn.x;
         acc[2] += rn.x * rn.x + rn.y * rn.y;
     }
-    tot_t<T> tot[4];
-    if (!last_block_total<4>(acc, R.part, gridDim.x, blockIdx.x, R.cnt + 3, sred, tot)) return;
+    tot_t<T> tot[3];
+    if (!last_block_total<3>(acc, R.part, gridDim.x, blockIdx.x, R.cnt + 3, sred, tot)) return;
     if (threadIdx.x != 0) return;
     finish_step(R.st, make_double2(tot[0], tot[1]), tot[2], is_init != 0);
 }
@@ -92,12 +96,12 @@ __global__ void __launch_bounds__(kNT) k_finish(int n3, int multi, const RhsVecs
 template <typename T>
 __global__ void __launch_bounds__(kNT) k_solve_begin(int n3, int multi, const RhsVecs<T>* __restrict__ rhs,
                                                      int resid_is_rhs) {
-    __shared__ double sred[sred_size<T, 4>()];
+    __shared__ double sred[sred_size<T, 1>()];
     const int b = blockIdx.y;
     const RhsVecs<T> R = rhs[b];
     if (rhs_done(R.st)) return;
     if (multi) n3 = 3 * R.N;  // a cross-lattice batch: this right-hand side's dipoles
-    acc_t<T> acc[4] = {0, 0, 0, 0};
+    acc_t<T> acc[1] = {0};
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n3; e += gridDim.x * blockDim.x) {
         const cx<T> v = R.E[e];
         acc[0] += v.x * v.x + v.y * v.y;
@@ -107,8 +111,8 @@ __global__ void __launch_bounds__(kNT) k_solve_begin(int n3, int multi, const Rh
             R.p[e] = v;
         }
     }
-    tot_t<T> tot[4];
-    if (!last_block_total<4>(acc, R.part, gridDim.x, blockIdx.x, R.cnt + 4, sred, tot)) return;
+    tot_t<T> tot[1];
+    if (!last_block_total<1>(acc, R.part, gridDim.x, blockIdx.x, R.cnt + 4, sred, tot)) return;
     if (threadIdx.x != 0) return;
     if constexpr (sizeof(T) == 4) {
         R.st->Enorm32 = sqrtf(tot[0].x);
@@ -134,14 +138,16 @@ __global__ void __launch_bounds__(kNT) k_chunk_end(const RhsVecs<float>* __restr
     if (threadIdx.x == 0) s_running = 0;
     for (int b = 0; b < nrhs; b++) {
         const RhsVecs<float> R = rhs[b];
-        StepIn in;
+        StepIn in = {};
         if (threadIdx.x == 0) in = load_step_in(R.st, slot);
         float2 tot[8];
         sum_partials<8>(R.part, prod_nblk, sred, tot);
-        if (threadIdx.x == 0 && in.status == ST_RUNNING) {
-            const StepEnd e = step_end_f32(in, tot);
-            write_step_end(R.st, e, slot);
-            if (e.stop == ST_RUNNING) s_running = 1;
+        if (threadIdx.x < 32 && __shfl_sync(0xffffffffu, in.status, 0) == ST_RUNNING) {
+            const StepEnd e = step_end_f32(in, sred);
+            if (threadIdx.x == 0) {
+                write_step_end(R.st, e, slot);
+                if (e.stop == ST_RUNNING) s_running = 1;
+            }
         }
         __syncthreads();  // sred is reused for the next right-hand side
     }
@@ -314,9 +320,9 @@ __global__ void k_green_fold(Geom g, const double2* __restrict__ full6, double2*
         const int fy = (int)(q / ((long long)g.Hx * g.Hz));
         const double2 v = full6[l * M + ((long long)fx * My + fy) * Mz + fz];
         const double2 w = make_double2(v.x * inv, v.y * inv);
-        green64[e] = w;
-        // FP32: planes of component pairs, [fy][fx][l / 2][fz][l % 2]
-        green32[((((long long)fy * g.Hx + fx) * 3 + l / 2) * g.Hz + fz) * 2 + (l & 1)] =
+        green64[fx * g.gs64.x + fy * g.gs64.y + fz * g.gs64.z + l * g.gs64.l] = w;
+        // FP32: planes of component pairs
+        green32[(fx * g.gs32.x + fy * g.gs32.y + fz * g.gs32.z + (l / 2) * g.gs32.l) * 2 + (l & 1)] =
             make_float2((float)w.x, (float)w.y);
     }
 }
@@ -569,21 +575,23 @@ int grid1d(long long n, int nt) {
     if (b > 152 * 16) b = 152 * 16;  // 16 resident blocks per SM on 152 SMs at most
     return (int)(b < 1 ? 1 : b);
 }
-// reductions over a vector: four entries per thread keeps the FP64 block
-// sums few while leaving enough threads to cover memory latency
-// blocks of a grid-stride reduction over n entries.  FP64 kernels: 4 entries
-// per thread, at most 8 blocks per SM (each block's FP64 block sum occupies
-// the narrow FP64 pipe).  FP32 kernels: 2 entries per thread for latency
-// hiding, and at most 8 per thread (their per-thread partials are FP32).
+// blocks of a grid-stride reduction over n entries.  FP64 kernels: at most 8
+// blocks per SM (each block's FP64 block sum occupies the narrow FP64 pipe), one
+// entry per thread below that: an FP64 chain of four entries a thread left most
+// of the FP64 pipes idle on small lattices.  FP32 kernels: 2 entries per thread
+// for latency hiding, and at most 8 per thread (their per-thread partials are
+// FP32).
 int grid_reduce(long long n, bool fp32) {
     long long b;
     if (fp32) {
         b = std::min((n + 2LL * kNT - 1) / (2LL * kNT), std::max(152LL * 16, (n + 8LL * kNT - 1) / (8LL * kNT)));
     } else {
-        b = (n + 4LL * kNT - 1) / (4LL * kNT);
-        if (b > 152 * 8) b = 152 * 8;
+        b = std::min((n + kNT - 1) / kNT, 152LL * 8);
     }
     return (int)(b < 1 ? 1 : b);
+}
+int grid_update(long long n) {
+    return (int)std::max(1LL, std::min((n + kNTUpdate - 1) / kNTUpdate, 152LL * 4));
 }
 
 size_t rowsmem(const AxisPlan& p) { return sizeof(double2) * (size_t)(p.M + 2 * row_lines(p) * pad_odd(p.M)); }
@@ -598,7 +606,7 @@ cudaError_t configure_kernels() {
     if (e == cudaSuccess) e = configure_pass_ct_xy();
     if (e == cudaSuccess) e = configure_pass_ct_xy2();
     if (e == cudaSuccess) e = configure_pass_zy();
-    if (e == cudaSuccess) e = configure_pass_dd();
+    if (e == cudaSuccess) e = configure_axes();
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPassSmem);
     if (e == cudaSuccess)
@@ -620,9 +628,10 @@ size_t max_pass_smem(const Geom& g) {
 int max_blocks_per_rhs(const Geom& g) {
     const int lz = std::min(z_lines<float>(g.pz.M), z_lines<double>(g.pz.M));
     int nz = (g.Nx * g.Ny + lz - 1) / lz;
-    int nv = std::max(grid_reduce(3LL * g.N, false), grid_reduce(3LL * g.N, true));
+    int nv = std::max(std::max(grid_reduce(3LL * g.N, false), grid_reduce(3LL * g.N, true)), grid_update(3LL * g.N));
     int nzy = 3 * g.Nx;  // fused z+y passes: one block per (x plane, component)
-    return std::max(nz, std::max(nv, nzy));
+    int nax = std::max(axis_sink_blocks(g, false), axis_sink_blocks(g, true));
+    return std::max(std::max(nz, nax), std::max(nv, nzy));
 }
 
 // ------------------------------------------------------------------ launchers
@@ -695,7 +704,9 @@ cudaError_t launch_aproduct(const Geom& g, int src, int snk, int nrhs, const Rhs
                             const cx<T>* twx, const cx<T>* twy, const cx<T>* twz, const int* cellmap, cx<T>* grid,
                             cudaStream_t stream, cudaEvent_t* ev, int slot) {
     const PassArgs<T> a{g, nrhs, rhs, green, twx, twy, twz, cellmap, grid, stream, slot, sink_blocks<T>(g)};
-    if (zy_fused(g, sizeof(T) == 4)) {
+    const ProductForm form = product_form(g, sizeof(T) == 4);
+    if (form >= FORM_AXES) return launch_axes<T>(src, snk, a, form == FORM_PLANE, ev);
+    if (form == FORM_FUSED_ZY) {
         cudaError_t err = cudaSuccess;
         if (ev) cudaEventRecord(ev[0], stream);
         if (!pass_zy<T>(PASS_ZFWD, src, a, &err)) return cudaErrorInvalidValue;
@@ -724,8 +735,18 @@ cudaError_t launch_aproduct(const Geom& g, int src, int snk, int nrhs, const Rhs
     return cudaSuccess;
 }
 
+// The x-first product where its lengths are compiled (FP32: in its plane form
+// where the plane fits a block, unless the shared-memory x pass is asked for),
+// else the z-y-x passes, fused where compiled.
+ProductForm product_form(const Geom& g, bool fp32) {
+    if (axes_lengths(g) && !g.passes && (!fp32 || g.x_form == 0)) return fp32 && axes_plane(g) ? FORM_PLANE : FORM_AXES;
+    return zy_fused(g, fp32) ? FORM_FUSED_ZY : FORM_PASSES;
+}
+
 template <typename T> int sink_blocks(const Geom& g) {
-    if (zy_fused(g, sizeof(T) == 4)) return 3 * g.Nx;  // one block per (x plane, component)
+    const ProductForm form = product_form(g, sizeof(T) == 4);
+    if (form >= FORM_AXES) return axis_sink_blocks(g, sizeof(T) == 4);
+    if (form == FORM_FUSED_ZY) return 3 * g.Nx;  // one block per (x plane, component)
     const int lz = z_lines<T>(g.pz.M);
     return (g.Nx * g.Ny + lz - 1) / lz;
 }
@@ -739,8 +760,8 @@ cudaError_t launch_chunk_end(const Geom& g, int nrhs, const RhsVecs<float>* rhs,
 
 template <typename T>
 cudaError_t launch_update(const Geom& g, int nrhs, const RhsVecs<T>* rhs, int is_init, cudaStream_t stream) {
-    const dim3 gr(grid_reduce(3LL * g.N, sizeof(T) == 4), nrhs);
-    k_update<T><<<gr, kNT, 0, stream>>>(3 * g.N, rhs, is_init);
+    const dim3 gr(grid_update(3LL * g.N), nrhs);
+    k_update<T><<<gr, kNTUpdate, 0, stream>>>(3 * g.N, rhs, is_init);
     return cudaGetLastError();
 }
 

@@ -66,20 +66,23 @@ __device__ __forceinline__ bool fp32_step_scalars(const RhsVecs<float>& R, int s
     __shared__ float2 s_sc[3];
     __shared__ int s_stop;
     if constexpr (SRC == SRC_PUPD_DEF) {
-        StepIn in;
+        StepIn in = {};
         if (threadIdx.x == 0) in = load_step_in(R.st, slot);
         float2 tot[8];
         sum_partials<8>(R.part, prod_nblk, scratch, tot);
-        if (threadIdx.x == 0) {
-            if (in.status != ST_RUNNING) {
-                s_stop = in.status;
+        if (threadIdx.x < 32) {  // the totals are in scratch
+            const int status = __shfl_sync(0xffffffffu, in.status, 0);
+            if (status != ST_RUNNING) {
+                if (threadIdx.x == 0) s_stop = status;
             } else {
-                const StepEnd e = step_end_f32(in, tot);
-                if (blockIdx.x == 0) write_step_end(R.st, e, slot);
-                s_sc[0] = e.zeta;
-                s_sc[1] = e.beta;
-                s_sc[2] = in.alpha;
-                s_stop = e.stop;
+                const StepEnd e = step_end_f32(in, scratch);
+                if (threadIdx.x == 0) {
+                    if (blockIdx.x == 0) write_step_end(R.st, e, slot);
+                    s_sc[0] = e.zeta;
+                    s_sc[1] = e.beta;
+                    s_sc[2] = in.alpha;
+                    s_stop = e.stop;
+                }
             }
         }
         __syncthreads();
@@ -233,43 +236,30 @@ __global__ void __launch_bounds__(kNT) k_ypass(Geom g, const RhsVecs<T>* __restr
 // xx, yy, zz even in all axes; xy odd in x,y; xz odd in x,z; yz odd in y,z
 __device__ __forceinline__ int fold(int k, int M) { return 2 * k > M ? M - k : k; }
 
-// the six components of one spectral point: 48 (FP32) or 96 (FP64) contiguous,
-// 16-byte aligned bytes, read as 16-byte vectors
-template <typename T>
-__device__ __forceinline__ void load_green6(const cx<T>* gg, cx<T>& a0, cx<T>& a1, cx<T>& a2, cx<T>& a3, cx<T>& a4,
-                                            cx<T>& a5) {
-    if constexpr (is_dd<T>) {
-        const float4* q = reinterpret_cast<const float4*>(gg);
-        a0 = dd2(__ldg(q)); a1 = dd2(__ldg(q + 1)); a2 = dd2(__ldg(q + 2));
-        a3 = dd2(__ldg(q + 3)); a4 = dd2(__ldg(q + 4)); a5 = dd2(__ldg(q + 5));
-    } else if constexpr (sizeof(cx<T>) == 8) {
-        const float4* q = reinterpret_cast<const float4*>(gg);
-        const float4 u = __ldg(q), v = __ldg(q + 1), w = __ldg(q + 2);
-        a0 = mk<T>(u.x, u.y); a1 = mk<T>(u.z, u.w);
-        a2 = mk<T>(v.x, v.y); a3 = mk<T>(v.z, v.w);
-        a4 = mk<T>(w.x, w.y); a5 = mk<T>(w.z, w.w);
-    } else {
-        a0 = __ldg(gg); a1 = __ldg(gg + 1); a2 = __ldg(gg + 2);
-        a3 = __ldg(gg + 3); a4 = __ldg(gg + 4); a5 = __ldg(gg + 5);
-    }
-}
-
-// The six components at folded point (fy, fx, fz).  FP64 and double-float
-// tables hold the six contiguously ([Hy][Hx][Hz][6]).  The FP32 table holds
-// them as three planes of component pairs ([Hy][Hx][3][Hz] float4: xx|xy,
-// xz|yy, yz|zz), so the threads of a warp that walk z read whole 128-byte
-// lines with each 16-byte load instead of a third of three lines each.
+// The six components at folded point (fy, fx, fz).  The FP32 table holds them as
+// three planes of component pairs (xx|xy, xz|yy, yz|zz), read as 16-byte values;
+// the FP64 and double-float tables hold 16-byte components.  The strides put the
+// axis that the threads of a warp walk innermost (GreenStride), so that a warp's
+// loads read whole lines.
 template <typename T>
 __device__ __forceinline__ void load_green(const cx<T>* green, const Geom& g, int fy, int fx, int fz, cx<T>& a0,
                                            cx<T>& a1, cx<T>& a2, cx<T>& a3, cx<T>& a4, cx<T>& a5) {
-    if constexpr (sizeof(cx<T>) == 8) {
-        const float4* q = reinterpret_cast<const float4*>(green) + ((long long)fy * g.Hx + fx) * 3 * g.Hz + fz;
-        const float4 u = __ldg(q), v = __ldg(q + g.Hz), w = __ldg(q + 2 * g.Hz);
+    const GreenStride& gs = sizeof(T) == 4 ? g.gs32 : g.gs64;
+    const long long at = fx * gs.x + fy * gs.y + fz * gs.z;
+    if constexpr (sizeof(T) == 4) {
+        const float4* q = reinterpret_cast<const float4*>(green) + at;
+        const float4 u = __ldg(q), v = __ldg(q + gs.l), w = __ldg(q + 2 * gs.l);
         a0 = mk<T>(u.x, u.y); a1 = mk<T>(u.z, u.w);
         a2 = mk<T>(v.x, v.y); a3 = mk<T>(v.z, v.w);
         a4 = mk<T>(w.x, w.y); a5 = mk<T>(w.z, w.w);
+    } else if constexpr (is_dd<T>) {
+        const float4* q = reinterpret_cast<const float4*>(green) + at;
+        a0 = dd2(__ldg(q)); a1 = dd2(__ldg(q + gs.l)); a2 = dd2(__ldg(q + 2 * gs.l));
+        a3 = dd2(__ldg(q + 3 * gs.l)); a4 = dd2(__ldg(q + 4 * gs.l)); a5 = dd2(__ldg(q + 5 * gs.l));
     } else {
-        load_green6<T>(green + (((long long)fy * g.Hx + fx) * g.Hz + fz) * 6, a0, a1, a2, a3, a4, a5);
+        const cx<T>* q = green + at;
+        a0 = __ldg(q); a1 = __ldg(q + gs.l); a2 = __ldg(q + 2 * gs.l);
+        a3 = __ldg(q + 3 * gs.l); a4 = __ldg(q + 4 * gs.l); a5 = __ldg(q + 5 * gs.l);
     }
 }
 
@@ -641,11 +631,16 @@ template <typename T, int SRC, int CH> struct GatherIn {
     static constexpr bool kPre = sizeof(T) == 4 && (SRC == SRC_IN || SRC == SRC_PUPD || SRC == SRC_TUPD ||
                                                     SRC == SRC_PUPD_DEF);
     cx<T> a[NL][CH];
-    __device__ __forceinline__ void load(const RhsVecs<T>& R, const long long (&o)[CH], const cx<T>* src) {
+    cx<T> pre[kPre ? CH : 1];
+    template <typename I>
+    __device__ __forceinline__ void load(const RhsVecs<T>& R, const I (&o)[CH], const cx<T>* src) {
 #pragma unroll
         for (int q = 0; q < CH; q++) {
             if (o[q] < 0) continue;
-            const long long i = o[q];
+            const I i = o[q];
+            if constexpr (kPre) {
+                if (R.pre) pre[q] = R.pre[i];
+            }
             if constexpr (SRC == SRC_PUPD_DEF) {
                 a[0][q] = R.Ap[i]; a[1][q] = R.r[i]; a[2][q] = R.p[i];
                 a[3][q] = R.t[i]; a[4][q] = R.At[i]; a[5][q] = R.P[i];
@@ -658,13 +653,14 @@ template <typename T, int SRC, int CH> struct GatherIn {
             }
         }
     }
-    __device__ __forceinline__ void combine(const RhsVecs<T>& R, const long long (&o)[CH], cx<T> (&v)[CH], cx<T> alpha,
+    template <typename I>
+    __device__ __forceinline__ void combine(const RhsVecs<T>& R, const I (&o)[CH], cx<T> (&v)[CH], cx<T> alpha,
                                             cx<T> beta, cx<T> zeta) const {
 #pragma unroll
         for (int q = 0; q < CH; q++) {
             v[q] = czero<T>();
             if (o[q] < 0) continue;
-            const long long i = o[q];
+            const I i = o[q];
             if constexpr (SRC == SRC_PUPD_DEF) {
                 // the previous step's update (DDAModel.cpp:226-230), then p (DDAModel.cpp:219)
                 const cx<T> Ap = a[0][q], r = a[1][q], p = a[2][q], t = a[3][q], At = a[4][q], P = a[5][q];
@@ -685,18 +681,11 @@ template <typename T, int SRC, int CH> struct GatherIn {
                 v[q] = a[0][q];
             }
             if constexpr (kPre) {  // the stored vectors stay unscaled; the grid gets D^-1 v
-                if (R.pre) v[q] = cmul<T>(v[q], R.pre[i]);
+                if (R.pre) v[q] = cmul<T>(v[q], pre[q]);
             }
         }
     }
 };
-template <typename T, int SRC, int CH>
-__device__ __forceinline__ void gather_chunk(const RhsVecs<T>& R, const long long (&o)[CH], cx<T> (&v)[CH],
-                                             const cx<T>* src, cx<T> alpha, cx<T> beta, cx<T> zeta) {
-    GatherIn<T, SRC, CH> in;
-    in.load(R, o, src);
-    in.combine(R, o, v, alpha, beta, zeta);
-}
 
 // Scatter of CH entries of one component (A v in val[q], dipole entry o[q] or
 // -1) with the sink's diagonal term, stores and dot-product terms.  All loads come before
@@ -1116,15 +1105,6 @@ template <typename T, int CM> struct PassLaunch {
             const int LZ = z_lines<T>(Mz);
             const dim3 grid((g.Nx * g.Ny + LZ - 1) / LZ, a.nrhs);
             const size_t sm = zsmem<T>(Mz);
-            if constexpr (is_dd<T>) {  // the double-float product forms residuals only
-                if (pass == PASS_ZFWD) {
-                    k_zfwd<T, SRC_P, CM><<<grid, kNT, sm, a.stream>>>(g, a.rhs, a.twz, a.cellmap, a.grid, a.slot,
-                                                                      a.prod_nblk);
-                } else {
-                    k_zinv<T, SRC_P, SNK_RES, CM><<<grid, kNT, sm, a.stream>>>(g, a.rhs, a.twz, a.cellmap, a.grid);
-                }
-                return cudaGetLastError();
-            }
             if (pass == PASS_ZFWD) {
                 switch (mode) {
                     case SRC_IN: k_zfwd<T, SRC_IN, CM><<<grid, kNT, sm, a.stream>>>(g, a.rhs, a.twz, a.cellmap, a.grid, a.slot, a.prod_nblk); break;
@@ -1174,10 +1154,6 @@ template <typename T, int CM> struct PassLaunch {
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPassSmem);
     }
     static cudaError_t configure_z() {
-        if constexpr (is_dd<T>) {
-            cudaError_t e = set_attr((const void*)k_zfwd<T, SRC_P, CM>);
-            return e != cudaSuccess ? e : set_attr((const void*)k_zinv<T, SRC_P, SNK_RES, CM>);
-        }
         const void* ks[] = {(const void*)k_zfwd<T, SRC_IN, CM>, (const void*)k_zfwd<T, SRC_PUPD, CM>,
                             (const void*)k_zfwd<T, SRC_TUPD, CM>, (const void*)k_zfwd<T, SRC_P, CM>,
                             (const void*)k_zfwd<T, SRC_PUPD_DEF, CM>, (const void*)k_zinv<T, SRC_TUPD, SNK_AT_DEF, CM>,
