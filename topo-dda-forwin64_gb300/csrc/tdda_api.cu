@@ -332,6 +332,19 @@ template <typename T> tdda_status dalloc_c(tdda_core* c, T** p, size_t count) {
 cudaMemcpyKind kind_in(int mem) { return mem == TDDA_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice; }
 cudaMemcpyKind kind_out(int mem) { return mem == TDDA_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost; }
 
+// Whether a kernel on `device` may read and write a caller's device vector in
+// place: memory of that device (or managed), 16-byte aligned.  Anything else a
+// copy can reach goes through a staging vector.
+bool kernel_may_use(const void* p, int device) {
+    cudaPointerAttributes at;
+    if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == device);
+}
+
 RhsVecs<double> vecs64(tdda_core* c, tdda_model* m, int slot) {
     RhsVecs<double> v{};
     v.P = m->P; v.E = m->E; v.r = m->r; v.r0 = m->r0; v.p = m->p; v.u = m->u; v.t = m->t;
@@ -1793,8 +1806,33 @@ tdda_status tdda_aproduct(tdda_core* c, int precision, const double* b, double* 
     }
     TDDA_TRY(set_device(c->device));
     const size_t n3 = 3 * (size_t)c->N;
+    const bool fp64 = precision == TDDA_FP64;
+    if (tdda::product_form(c->g, !fp64) >= tdda::FORM_AXES) {
+        // the x kernels read and write FP64 vectors themselves: a device caller's in
+        // place where a kernel may touch them, else the core's staging vectors
+        const double2* in = reinterpret_cast<const double2*>(b);
+        double2* out = reinterpret_cast<double2*>(y);
+        const bool own_in = mem == TDDA_MEM_DEVICE && kernel_may_use(b, c->device);
+        const bool own_out = mem == TDDA_MEM_DEVICE && kernel_may_use(y, c->device);
+        if (!own_in) {
+            TDDA_CK(cudaMemcpyAsync(c->vin64, b, sizeof(double2) * n3, kind_in(mem), c->stream));
+            in = c->vin64;
+        }
+        if (!own_out) out = c->vout64;
+        count_launches(fp64 ? product_kernels<double>(c) : product_kernels<float>(c));
+        if (fp64) {
+            TDDA_CK(tdda::launch_aproduct_ext<double>(c->g, c->rhs64 + c->max_rhs, in, out, c->green64, c->tw64[0],
+                                                      c->tw64[1], c->tw64[2], c->cellmap, c->grid64, c->stream));
+        } else {
+            TDDA_CK(tdda::launch_aproduct_ext<float>(c->g, c->rhs32 + c->max_rhs, in, out, c->green32, c->tw32[0],
+                                                     c->tw32[1], c->tw32[2], c->cellmap, c->grid32, c->stream));
+        }
+        if (!own_out) TDDA_CK(cudaMemcpyAsync(y, out, sizeof(double2) * n3, kind_out(mem), c->stream));
+        TDDA_CK(cudaStreamSynchronize(c->stream));
+        return TDDA_OK;
+    }
     TDDA_CK(cudaMemcpyAsync(c->vin64, b, sizeof(double2) * n3, kind_in(mem), c->stream));
-    if (precision == TDDA_FP64) {
+    if (fp64) {
         TDDA_CK(aprod<double>(c, tdda::SRC_IN, tdda::SNK_OUT, 1, c->rhs64 + c->max_rhs));
     } else {
         TDDA_CK1(tdda::launch_to_f32((int)n3, c->vin64, c->vin32, c->stream));

@@ -88,11 +88,12 @@ template <int R, int SIGN, typename T> __device__ __forceinline__ void twiddle(c
 // SoA and their lines component-major; FP64 vectors are AoS and their lines
 // cell-major, so that consecutive lines are consecutive entries of either.
 template <typename T> constexpr bool kSoa = sizeof(T) == 4;
-// entry of the dipole vectors at cell (x, line), or -1; 32 bits hold it (a box
-// has at most 2^28 cells)
-template <typename T> __device__ __forceinline__ int line_entry(const Lat& L, int NC, int x, int cell, int c) {
+// entry of the dipole vectors (of an AoS vector: AOS) at cell (x, line), or -1;
+// 32 bits hold it (a box has at most 2^28 cells)
+template <typename T, bool AOS = false>
+__device__ __forceinline__ int line_entry(const Lat& L, int NC, int x, int cell, int c) {
     const int i = L.dense ? x * NC + cell : L.cellmap[x * NC + cell];
-    return i >= 0 ? (int)vec_index<T>(i, c, L.N) : -1;
+    return i < 0 ? -1 : AOS ? 3 * i + c : (int)vec_index<T>(i, c, L.N);
 }
 // offset of a line in one kx plane of the work grid whose components (SoA) are
 // `rows` rows of Nz entries
@@ -268,7 +269,7 @@ template <typename T, int M, int CT> struct XTile {
 // the diagonal term, the stores and the dot-product terms from A v in val.
 template <typename T, int SRC, int SNK, int CH> struct SinkIn {
     cx<T> vv[CH], al[CH], q2[CH];
-    static constexpr bool kV = SNK != SNK_OUT, kQ = SNK == SNK_AP || SNK == SNK_AT_DEF || SNK == SNK_RES;
+    static constexpr bool kV = SNK != SNK_OUT && SNK != SNK_EXT, kQ = SNK == SNK_AP || SNK == SNK_AT_DEF || SNK == SNK_RES;
     bool unit;  // a Jacobi-preconditioned product adds 1 v (RhsVecs::pre)
     __device__ __forceinline__ void load(const RhsVecs<T>& R, const int (&o)[CH]) {
         const cx<T>* vsrc = SRC == SRC_TUPD ? R.t : (SRC == SRC_P ? R.P : R.p);
@@ -285,11 +286,13 @@ template <typename T, int SRC, int SNK, int CH> struct SinkIn {
     }
     template <int NV>
     __device__ __forceinline__ void store(const RhsVecs<T>& R, const int (&o)[CH], const cx<T>* val,
-                                          acc_t<T> (&acc)[NV]) const {
+                                          acc_t<T> (&acc)[NV], double2* ext) const {
 #pragma unroll
         for (int q = 0; q < CH; q++) {
             if (o[q] < 0) continue;
-            if constexpr (SNK == SNK_OUT) {
+            if constexpr (SNK == SNK_EXT) {
+                ext[o[q]] = make_double2((double)val[q].x, (double)val[q].y);
+            } else if constexpr (SNK == SNK_OUT) {
                 R.Ap[o[q]] = val[q];
             } else {
                 const cx<T> t = vv[q], w = cadd<T>(val[q], unit ? t : cmul<T>(t, al[q]));
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(axis_threads<M, CT>(), axis_minb<M, CT>()) k_x
                                                                 const cx<T>* __restrict__ twx,
                                                                 const int* __restrict__ cellmap,
                                                                 cx<T>* __restrict__ grid, int pitch_rows, int slot,
-                                                                int prod_nblk) {
+                                                                int prod_nblk, const double2* in_ext) {
     using A = AxisXY<M>;
     using TL = XTile<T, M, CT>;
     constexpr bool kStep32 = sizeof(T) == 4 && (SRC == SRC_PUPD_DEF || SRC == SRC_TUPD);
@@ -373,10 +376,13 @@ __global__ void __launch_bounds__(axis_threads<M, CT>(), axis_minb<M, CT>()) k_x
 #pragma unroll
         for (int r = 0; r < RH; r++) {
             const int x = j + R2 * r;
-            o[r] = j < R2 && line < NL && x < L.Nx ? line_entry<T>(L, NC, x, cell, c) : -1;
+            o[r] = j < R2 && line < NL && x < L.Nx ? line_entry<T, SRC == SRC_EXT>(L, NC, x, cell, c) : -1;
         }
         cx<T> v[R1];
-        if constexpr (is_dd<T>) {
+        if constexpr (SRC == SRC_EXT) {
+#pragma unroll
+            for (int r = 0; r < RH; r++) v[r] = o[r] >= 0 ? from_d<T>(in_ext[o[r]]) : czero<T>();
+        } else if constexpr (is_dd<T>) {
 #pragma unroll
             for (int r = 0; r < RH; r++) v[r] = o[r] >= 0 ? ldv<T>(src, o[r]) : czero<T>();
         } else {
@@ -421,7 +427,8 @@ template <typename T, int SRC, int SNK, int M, int CT>
 __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const RhsVecs<T>* __restrict__ rhs,
                                                                   const cx<T>* __restrict__ twx,
                                                                   const int* __restrict__ cellmap,
-                                                                  const cx<T>* __restrict__ grid, int pitch_rows) {
+                                                                  const cx<T>* __restrict__ grid, int pitch_rows,
+                                                                  double2* out_ext) {
     using A = AxisXY<M>;
     using TL = XTile<T, M, CT>;
     constexpr int R1 = A::R1, R2 = A::R2, RH = A::RH, LX = A::LX, NT = sink_threads<T, M, CT>();
@@ -429,7 +436,7 @@ __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<T>* stw = reinterpret_cast<cx<T>*>(smem_raw);
     cx<T>* s = stw + M;
-    constexpr bool kSums = SNK != SNK_OUT && SNK != SNK_ALB;
+    constexpr bool kSums = SNK != SNK_OUT && SNK != SNK_ALB && SNK != SNK_EXT;
     __shared__ double sred[!kSums ? 1 : sizeof(T) == 4 ? NV * (NT / 32) : NV * NT];
     const int b = blockIdx.y;
     const RhsVecs<T> R = rhs[b];
@@ -466,7 +473,7 @@ __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const
 #pragma unroll
             for (int r = 0; r < RH; r++) {
                 const int x = j + R2 * r;
-                o[r] = j < R2 && line < NL && x < L.Nx ? line_entry<T>(L, NC, x, cell, c) : -1;
+                o[r] = j < R2 && line < NL && x < L.Nx ? line_entry<T, SNK == SNK_EXT>(L, NC, x, cell, c) : -1;
             }
             SinkIn<T, SRC, SNK, RH> in;
             in.load(R, o);
@@ -476,7 +483,7 @@ __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const
 #pragma unroll
                 for (int q = 0; q < R1; q++) v[q] = s[j * TL::JS + q * CT + l];
                 Bfly<R1, +1, T>::run(v);
-                in.template store<NV>(R, o, v, acc);
+                in.template store<NV>(R, o, v, acc, out_ext);
             }
         } else {
             __syncthreads();
@@ -496,7 +503,7 @@ __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const
                 const cx<T> v = s[(x % R2) * TL::JS + (x / R2) * CT + le];
                 SinkIn<T, SRC, SNK, 1> in;
                 in.load(R, o);
-                in.template store<NV>(R, o, &v, acc);
+                in.template store<NV>(R, o, &v, acc, out_ext);
             }
         }
     } else {
@@ -1105,7 +1112,7 @@ template <typename T, int M> struct AxisLaunch {
         const unsigned per = (unsigned)((tiles + room - 1) / room);
         grid.x = (grid.x + per - 1) / per;
         return launch_axis(a, k_xfwd<T, SRC, M, CT>, grid, axis_threads<M, CT>(), XTile<T, M, CT>::smem, a.rhs, a.twx,
-                           a.cellmap, a.grid, rows, a.slot, a.prod_nblk);
+                           a.cellmap, a.grid, rows, a.slot, a.prod_nblk, a.in);
     }
     template <int SRC> static cudaError_t fwd(const PassArgs<T>& a, int rows) {
         if constexpr (sizeof(T) == 4) {
@@ -1115,7 +1122,7 @@ template <typename T, int M> struct AxisLaunch {
     }
     template <int SRC, int SNK, int CT> static cudaError_t inv1(const PassArgs<T>& a, int rows) {
         return launch_axis(a, k_xinv<T, SRC, SNK, M, CT>, lines(a, CT), sink_threads<T, M, CT>(), XTile<T, M, CT>::smem,
-                           a.rhs, a.twx, a.cellmap, (const cx<T>*)a.grid, rows);
+                           a.rhs, a.twx, a.cellmap, (const cx<T>*)a.grid, rows, a.out);
     }
     template <int SRC, int SNK> static cudaError_t inv(const PassArgs<T>& a, int rows) {
         if constexpr (sizeof(T) == 4) {
@@ -1136,14 +1143,24 @@ template <typename T, int M> struct AxisLaunch {
         if constexpr (is_dd<T>) {  // the double-float product forms residuals only
             return op == AXIS_XFWD ? fwd<SRC_P>(a, rows) : inv<SRC_P, SNK_RES>(a, rows);
         } else if constexpr (sizeof(T) == 4) {  // products and the deferred step
-            if (op == AXIS_XFWD)
-                return mode == SRC_IN ? fwd<SRC_IN>(a, rows)
-                                      : mode == SRC_TUPD ? fwd<SRC_TUPD>(a, rows) : fwd<SRC_PUPD_DEF>(a, rows);
-            return mode == SNK_OUT ? inv<SRC_IN, SNK_OUT>(a, rows)
-                                   : mode == SNK_AP ? inv<SRC_PUPD, SNK_AP>(a, rows) : inv<SRC_TUPD, SNK_AT_DEF>(a, rows);
+            if (op == AXIS_XFWD) {
+                switch (mode) {
+                    case SRC_EXT: return fwd<SRC_EXT>(a, rows);
+                    case SRC_IN: return fwd<SRC_IN>(a, rows);
+                    case SRC_TUPD: return fwd<SRC_TUPD>(a, rows);
+                    default: return fwd<SRC_PUPD_DEF>(a, rows);
+                }
+            }
+            switch (mode) {
+                case SNK_EXT: return inv<SRC_EXT, SNK_EXT>(a, rows);
+                case SNK_OUT: return inv<SRC_IN, SNK_OUT>(a, rows);
+                case SNK_AP: return inv<SRC_PUPD, SNK_AP>(a, rows);
+                default: return inv<SRC_TUPD, SNK_AT_DEF>(a, rows);
+            }
         } else {
             if (op == AXIS_XFWD) {
                 switch (mode) {
+                    case SRC_EXT: return fwd<SRC_EXT>(a, rows);
                     case SRC_IN: return fwd<SRC_IN>(a, rows);
                     case SRC_PUPD: return fwd<SRC_PUPD>(a, rows);
                     case SRC_TUPD: return fwd<SRC_TUPD>(a, rows);
@@ -1151,6 +1168,7 @@ template <typename T, int M> struct AxisLaunch {
                 }
             }
             switch (mode) {
+                case SNK_EXT: return inv<SRC_EXT, SNK_EXT>(a, rows);
                 case SNK_OUT: return inv<SRC_IN, SNK_OUT>(a, rows);
                 case SNK_ALB: return inv<SRC_IN, SNK_ALB>(a, rows);
                 case SNK_AP: return inv<SRC_PUPD, SNK_AP>(a, rows);

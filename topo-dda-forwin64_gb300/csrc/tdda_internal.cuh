@@ -181,6 +181,7 @@ enum SrcMode : int {
     SRC_PUPD_DEF = 4,  // apply the deferred update of the previous step
                        // (u = zeta Ap, P += alpha p + zeta r - alpha u,
                        // r = t - zeta At), then p = r + beta (p - u)
+    SRC_EXT = 5,     // v = PassArgs::in, an FP64 AoS vector (plain products, x-first only)
 };
 // what the last z-pass does with A v
 enum SnkMode : int {
@@ -192,6 +193,7 @@ enum SnkMode : int {
     SNK_AT_DEF = 5,  // At = A t + al t; zeta, and r0.r and |r|^2 of r = t - zeta At from
                      // r0.t, r0.At, t.t, At.t, At.At; the step logic of launch_update;
                      // the update of P and r is left pending (SRC_PUPD_DEF, launch_finish)
+    SNK_EXT = 6,     // PassArgs::out = A v, an FP64 AoS vector (plain products, x-first only)
 };
 
 // -------------------------------------------------------------- pass dispatch
@@ -212,6 +214,9 @@ template <typename T> struct PassArgs {
     cudaStream_t stream;
     int slot;       // FP32 deferred step: parity of the step (state slots)
     int prod_nblk;  // FP32 deferred step: blocks of the sink pass whose partials this gather reads
+    // SRC_EXT / SNK_EXT: the caller's vectors, read and written by the x kernels
+    const double2* in = nullptr;
+    double2* out = nullptr;
 };
 // mode: SrcMode for PASS_ZFWD, SnkMode for PASS_ZINV, unused otherwise
 template <typename T> cudaError_t pass_generic(int pass, int mode, const PassArgs<T>& a);
@@ -299,6 +304,12 @@ cudaError_t launch_aproduct(const Geom& g, int src, int snk, int nrhs, const Rhs
                             const cx<T>* green, const cx<T>* twx, const cx<T>* twy, const cx<T>* twz,
                             const int* cellmap, cx<T>* grid, cudaStream_t stream, cudaEvent_t* ev = nullptr,
                             int slot = 0);
+// y = A_offdiag b for FP64 AoS vectors b and y (device memory, 16-byte aligned;
+// they may overlap), at precision T, without staging copies; the x-first forms only
+template <typename T>
+cudaError_t launch_aproduct_ext(const Geom& g, const RhsVecs<T>* rhs, const double2* b, double2* y, const cx<T>* green,
+                                const cx<T>* twx, const cx<T>* twy, const cx<T>* twz, const int* cellmap,
+                                cx<T>* grid, cudaStream_t stream);
 // blocks of the last pass of an A-product at precision T (the producer of the
 // dot-product partials)
 template <typename T> int sink_blocks(const Geom& g);

@@ -735,6 +735,16 @@ cudaError_t launch_aproduct(const Geom& g, int src, int snk, int nrhs, const Rhs
     return cudaSuccess;
 }
 
+template <typename T>
+cudaError_t launch_aproduct_ext(const Geom& g, const RhsVecs<T>* rhs, const double2* b, double2* y, const cx<T>* green,
+                                const cx<T>* twx, const cx<T>* twy, const cx<T>* twz, const int* cellmap,
+                                cx<T>* grid, cudaStream_t stream) {
+    const ProductForm form = product_form(g, sizeof(T) == 4);
+    if (form < FORM_AXES) return cudaErrorInvalidValue;
+    const PassArgs<T> a{g, 1, rhs, green, twx, twy, twz, cellmap, grid, stream, 0, 0, b, y};
+    return launch_axes<T>(SRC_EXT, SNK_EXT, a, form == FORM_PLANE, nullptr);
+}
+
 // The x-first product where its lengths are compiled (FP32: in its plane form
 // where the plane fits a block, unless the shared-memory x pass is asked for),
 // else the z-y-x passes, fused where compiled.
@@ -883,6 +893,9 @@ template <typename T> cudaError_t launch_zero(long long n, cx<T>* v, cudaStream_
     template cudaError_t launch_aproduct<T>(const Geom&, int, int, int, const RhsVecs<T>*, const cx<T>*,          \
                                             const cx<T>*, const cx<T>*, const cx<T>*, const int*, cx<T>*,         \
                                             cudaStream_t, cudaEvent_t*, int);                                      \
+    template cudaError_t launch_aproduct_ext<T>(const Geom&, const RhsVecs<T>*, const double2*, double2*,          \
+                                                const cx<T>*, const cx<T>*, const cx<T>*, const cx<T>*,           \
+                                                const int*, cx<T>*, cudaStream_t);                                 \
     template int sink_blocks<T>(const Geom&);                                                                      \
     template cudaError_t launch_finish<T>(const Geom&, int, const RhsVecs<T>*, cudaStream_t);                      \
     template cudaError_t launch_solve_begin<T>(const Geom&, int, const RhsVecs<T>*, cudaStream_t);                 \
