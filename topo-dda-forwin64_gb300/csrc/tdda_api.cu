@@ -378,6 +378,7 @@ tdda::AlphaParams alpha_params(const tdda_model* m) {
     std::memset(&ap, 0, sizeof(ap));
     ap.a1c = 3 * std::pow(c->d, 3) / (4 * kPi);
     ap.d3 = std::pow(c->d, 3);
+    ap.rd3 = 1.0 / ap.d3;
     ap.Kd2 = std::pow(c->K * c->d, 2);
     ap.rad = (2.0 / 3.0) * std::pow(c->K * c->d, 3);
     ap.S = std::pow(m->nE0[0] * m->nK[0], 2) + std::pow(m->nE0[1] * m->nK[1], 2) + std::pow(m->nE0[2] * m->nK[2], 2);

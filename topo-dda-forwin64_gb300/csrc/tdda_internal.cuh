@@ -354,6 +354,7 @@ constexpr int kMaxMaterials = 16;
 struct AlphaParams {
     double a1c;   // 3 d^3 / (4 pi)
     double d3;    // d^3
+    double rd3;   // 1 / d^3
     double Kd2;   // (K d)^2
     double rad;   // (2/3) (K d)^3
     double S;     // sum_i (nE0_i nK_i)^2

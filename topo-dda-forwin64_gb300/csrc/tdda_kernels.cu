@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kNT) k_chunk_end(const RhsVecs<float>* __restr
 // DDAModel.cpp:530-565), FP64.  Pass 1: block (b, p) sums the dipoles
 // i = b*nt + t, b*nt + t + gridDim.x*nt, ... for point p in a fixed order and
 // writes its three complex partials; pass 2 adds the nb partials of each point
-// in block order and subtracts them from the incident field.
+// in a fixed order and subtracts them from the incident field.
 __global__ void __launch_bounds__(kNT) k_field_partial(int N, const int* __restrict__ R, double d, double K,
                                                        Interaction it, const double2* __restrict__ P,
                                                        const double* __restrict__ pts, double2* __restrict__ part) {
@@ -200,22 +200,30 @@ __global__ void __launch_bounds__(kNT) k_field_partial(int N, const int* __restr
     }
 }
 
+// One warp per point: lane l adds the partials l, l + 32, ... and a shuffle tree
+// the lanes (one thread adding all partials of a point in turn was a chain of
+// dependent loads: the density objective of an 80x80x20 box 165 -> 12 us)
 __global__ void k_field_sum(int npts, int nb, const double2* __restrict__ part, const double* __restrict__ pts,
                             double3 nK, double3 nE0, double E0, double K, double2* __restrict__ E) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int p = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
     if (p >= npts) return;
+    double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int b = lane; b < nb; b += 32) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const double2 v = part[((long long)p * nb + b) * 3 + j];
+            s[2 * j] += v.x;
+            s[2 * j + 1] += v.y;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 6; j++) s[j] += __shfl_down_sync(0xffffffffu, s[j], o);
+    if (lane) return;
     double sn, cs;
     sincos(K * (nK.x * pts[3 * p] + nK.y * pts[3 * p + 1] + nK.z * pts[3 * p + 2]), &sn, &cs);
     const double amp[3] = {E0 * nE0.x, E0 * nE0.y, E0 * nE0.z};
-    for (int j = 0; j < 3; j++) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int b = 0; b < nb; b++) {
-            const double2 v = part[((long long)p * nb + b) * 3 + j];
-            s.x += v.x;
-            s.y += v.y;
-        }
-        E[3 * p + j] = make_double2(amp[j] * cs - s.x, amp[j] * sn - s.y);
-    }
+    for (int j = 0; j < 3; j++) E[3 * p + j] = make_double2(amp[j] * cs - s[2 * j], amp[j] * sn - s[2 * j + 1]);
 }
 
 // Periodic lattice (AProductCore.cpp:251-536): the tensor at offset o is the
@@ -389,7 +397,23 @@ __global__ void __launch_bounds__(kNT) k_fft_cols(double2* __restrict__ data, in
 __device__ __forceinline__ double2 dadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 dscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 
-// eps and al = 1 / alpha_LDR(eps) of one density (DDAModel.cpp:54-63, tools.cpp:617-630)
+// a / b by one complex reciprocal (Smith's algorithm): two FP64 divisions
+// instead of three, and one reciprocal serves several numerators
+__device__ __forceinline__ double2 crecip(double2 b) {
+    if (fabs(b.x) >= fabs(b.y)) {
+        const double r = b.y / b.x, w = 1.0 / (b.x + b.y * r);
+        return make_double2(w, -r * w);
+    }
+    const double r = b.x / b.y, w = 1.0 / (b.x * r + b.y);
+    return make_double2(r * w, -w);
+}
+
+// eps and al = 1 / alpha_LDR(eps) of one density (DDAModel.cpp:54-63, tools.cpp:617-630).
+// alpha = a1 / (1 + (a1 / d^3) t) with a1 = c (eps - 1) / (eps + 2), c = 3 d^3 / (4 pi), and
+// t = (b1 + eps b2 + eps b3 S) (K d)^2 - i (2/3) (K d)^3, so 1 / alpha = 1 / a1 + t / d^3: one
+// complex division (an FP64 division is some ten FP64 instructions, and 11 of them were most
+// of this kernel: 221,184 dipoles 75 -> 26 us).  1 / a1 is finite at the pole eps = -2, where
+// alpha and the internal field are not: al stays NaN there.
 __device__ __forceinline__ void model_alpha_one(double v, const AlphaParams& ap, double2& eps, double2& inv) {
     const double b1 = -1.891531, b2 = 0.1648469, b3 = -1.7700004;  // LDR coefficients (tools.cpp:618-620)
     int lf = (int)floor(v);
@@ -400,14 +424,12 @@ __device__ __forceinline__ void model_alpha_one(double v, const AlphaParams& ap,
     const double2 mf = ap.mat[lf], mn = ap.mat[ln];
     const double w = v - (double)lf;
     eps = make_double2(mf.x + w * (mn.x - mf.x), mf.y + w * (mn.y - mf.y));
-    // a1 = (3 d^3 / (4 pi)) (eps - 1) / (eps + 2)
-    const double2 a1 = cdiv(dscale(make_double2(eps.x - 1.0, eps.y), ap.a1c), make_double2(eps.x + 2.0, eps.y));
-    // result = 1 + (a1 / d^3) ((b1 + eps b2 + eps b3 S) (K d)^2 - i (2/3)(K d)^3)
+    // 1 / a1 = (eps + 2) / (c (eps - 1))
+    const double2 ra = dmul(make_double2(eps.x + 2.0, eps.y), crecip(dscale(make_double2(eps.x - 1.0, eps.y), ap.a1c)));
     const double2 q = dadd(dadd(make_double2(b1, 0.0), dscale(eps, b2)), dscale(dscale(eps, b3), ap.S));
     const double2 t = make_double2(q.x * ap.Kd2, q.y * ap.Kd2 - ap.rad);
-    const double2 res = dadd(make_double2(1.0, 0.0), dmul(make_double2(a1.x / ap.d3, a1.y / ap.d3), t));
-    const double2 alpha = cdiv(a1, res);
-    inv = cdiv(make_double2(1.0, 0.0), alpha);
+    inv = make_double2(fma(t.x, ap.rd3, ra.x), fma(t.y, ap.rd3, ra.y));
+    if (eps.x == -2.0 && eps.y == 0.0) inv.x = inv.y = nan("");
 }
 
 __global__ void k_to_dd(long long n, const double2* __restrict__ src, dd2* __restrict__ dst) {
@@ -464,24 +486,46 @@ __device__ __forceinline__ double2 dal_drho(double2 eps, double v, const AlphaPa
     return dmul(dal, make_double2(ap.mat[1].x - ap.mat[0].x, ap.mat[1].y - ap.mat[0].y));
 }
 
-__global__ void k_density_gradient(int nparam, const int* __restrict__ off, const int* __restrict__ dip,
-                                   const double2* __restrict__ P, const double2* __restrict__ eps,
-                                   const double* __restrict__ diel_old, AlphaParams ap, GradArgs ga,
-                                   double* __restrict__ s) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nparam) return;
+// The terms of a block's kGradParams parameters are formed by all of its
+// threads, list entry by list entry, into shared memory, and one thread per
+// parameter adds its own in list order (one thread forming and adding all terms
+// of a parameter: 6400 parameters of 20 dipoles 240 -> 62 us).
+constexpr int kGradParams = 32, kGradChunk = 256;
+__global__ void __launch_bounds__(128) k_density_gradient(int nparam, const int* __restrict__ off,
+                                                          const int* __restrict__ dip, const double2* __restrict__ P,
+                                                          const double2* __restrict__ eps,
+                                                          const double* __restrict__ diel_old, AlphaParams ap,
+                                                          GradArgs ga, double* __restrict__ s) {
+    __shared__ double term[3 * kGradChunk];
+    const int i0 = blockIdx.x * kGradParams, i1 = min(nparam, i0 + kGradParams);
+    const int mine = i0 + threadIdx.x;
+    const bool sums = threadIdx.x < kGradParams && mine < nparam;
+    const int from = sums ? off[mine] : 0, to = sums ? off[mine + 1] : 0;
+    const int q1 = off[i1];
     double acc = 0.0;
-    for (int q = off[i]; q < off[i + 1]; q++) {
-        const int j = dip[q];
-        for (int c = 0; c < 3; c++) {
-            const int e = 3 * j + c;
-            double2 lam = make_double2(0.0, 0.0);
-            for (int k = 0; k < ga.nadj; k++) lam = dadd(lam, dmul(ga.coef[k], ga.lam[k][e]));
-            const double2 t = dmul(dmul(lam, dal_drho(eps[e], diel_old[e], ap)), P[e]);
-            acc += t.x;
+    for (int q0 = off[i0], qe; q0 < q1; q0 = qe) {
+        qe = q0 + min(q1 - q0, kGradChunk);
+        for (int q = q0 + threadIdx.x; q < qe; q += blockDim.x) {
+            const int j = dip[q];
+            double2 da = make_double2(0.0, 0.0), last = da;
+            double vlast = 0.0;
+            for (int c = 0; c < 3; c++) {
+                const int e = 3 * j + c;
+                const double2 ee = eps[e];
+                const double v = diel_old[e];
+                if (c == 0 || !(ee.x == last.x && ee.y == last.y && v == vlast)) da = dal_drho(ee, v, ap);
+                last = ee, vlast = v;
+                double2 lam = make_double2(0.0, 0.0);
+                for (int k = 0; k < ga.nadj; k++) lam = dadd(lam, dmul(ga.coef[k], ga.lam[k][e]));
+                term[3 * (q - q0) + c] = dmul(dmul(lam, da), P[e]).x;
+            }
         }
+        __syncthreads();
+        for (int q = max(from, q0); q < min(to, qe); q++)
+            for (int c = 0; c < 3; c++) acc += term[3 * (q - q0) + c];
+        __syncthreads();
     }
-    s[i] = acc;
+    if (sums) s[mine] = acc;
 }
 
 __global__ void k_model_incident(int N, const int* __restrict__ R, double3 nK, double3 nE0, double E0, double K,
@@ -497,10 +541,20 @@ __global__ void k_model_incident(int N, const int* __restrict__ R, double3 nK, d
 }
 
 // ------------------------------------------------------------ small kernels
+// One thread per dipole: the three entries normally hold the same eps, whose
+// factor 3 / (2 + eps) is formed once (221,184 dipoles: 96 -> 30 us)
 __global__ void k_einternal(int n3, const double2* al, const double2* P, const double2* diel, double2* Ein) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n3; e += gridDim.x * blockDim.x) {
-        const double2 lf = make_double2((2.0 + diel[e].x) / 3.0, diel[e].y / 3.0);
-        Ein[e] = cdiv(dmul(al[e], P[e]), lf);
+    const int n = n3 / 3;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double2 last = make_double2(0.0, 0.0), w = last;
+        for (int c = 0; c < 3; c++) {
+            const int e = 3 * i + c;
+            const double2 eps = diel[e];
+            if (c == 0 || !(eps.x == last.x && eps.y == last.y))
+                w = dscale(crecip(make_double2(2.0 + eps.x, eps.y)), 3.0);
+            last = eps;
+            Ein[e] = dmul(dmul(al[e], P[e]), w);
+        }
     }
 }
 // FP64 AoS vector -> FP32 SoA vector (the layouts of RhsVecs<double> and <float>)
@@ -818,7 +872,7 @@ cudaError_t launch_field_at(int N, const int* R, double d, double K, const Inter
         k_field_partial<<<dim3(nb, np), kNT, 0, stream>>>(N, R, d, K, it, P, pts + 3LL * p0, pp);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        k_field_sum<<<grid1d(np, 128), 128, 0, stream>>>(np, nb, pp, pts + 3LL * p0, nK, nE0, E0, K, E + 3LL * p0);
+        k_field_sum<<<(32 * np + 127) / 128, 128, 0, stream>>>(np, nb, pp, pts + 3LL * p0, nK, nE0, E0, K, E + 3LL * p0);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -827,7 +881,7 @@ cudaError_t launch_field_at(int N, const int* R, double d, double K, const Inter
 
 cudaError_t launch_einternal(int n3, const double2* al, const double2* P, const double2* diel, double2* Ein,
                              cudaStream_t stream) {
-    k_einternal<<<grid1d(n3, kNT), kNT, 0, stream>>>(n3, al, P, diel, Ein);
+    k_einternal<<<grid1d(n3 / 3, 128), 128, 0, stream>>>(n3, al, P, diel, Ein);
     return cudaGetLastError();
 }
 cudaError_t launch_scan(long long n, const double* v, int mode, double hi, unsigned int* flag, cudaStream_t stream) {
@@ -838,13 +892,13 @@ cudaError_t launch_scan(long long n, const double* v, int mode, double hi, unsig
 }
 cudaError_t launch_model_alpha(int n3, const double* diel_old, const AlphaParams& ap, double2* diel, double2* al,
                                float2* fal, cudaStream_t stream) {
-    k_model_alpha<<<grid1d(n3 / 3, kNT), kNT, 0, stream>>>(n3, diel_old, ap, diel, al, fal);
+    k_model_alpha<<<grid1d(n3 / 3, 128), 128, 0, stream>>>(n3, diel_old, ap, diel, al, fal);
     return cudaGetLastError();
 }
 cudaError_t launch_density_gradient(int nparam, const int* off, const int* dip, const double2* P, const double2* eps,
                                     const double* diel_old, const AlphaParams& ap, const GradArgs& ga, double* s,
                                     cudaStream_t stream) {
-    k_density_gradient<<<grid1d(nparam, 128), 128, 0, stream>>>(nparam, off, dip, P, eps, diel_old, ap, ga, s);
+    k_density_gradient<<<(nparam + kGradParams - 1) / kGradParams, 128, 0, stream>>>(nparam, off, dip, P, eps, diel_old, ap, ga, s);
     return cudaGetLastError();
 }
 cudaError_t launch_model_incident(int N, const int* R, double3 nK, double3 nE0, double E0, double K, double d,
