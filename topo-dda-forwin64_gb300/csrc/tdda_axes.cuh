@@ -495,15 +495,31 @@ __global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const
 #pragma unroll
                 for (int r = 0; r < RH; r++) s[j * TL::JS + r * CT + l] = v[r];
             }
-            __syncthreads();
-            for (int e = threadIdx.x; e < LX * CT; e += NT) {  // cell x = j + R2 r of line l0 + l
-                const int x = e / CT, le = e % CT, ln = l0 + le;
-                int o[1];
-                o[0] = ln < NL && x < L.Nx ? line_entry<T>(L, NC, x, ln / 3, ln % 3) : -1;
-                const cx<T> v = s[(x % R2) * TL::JS + (x / R2) * CT + le];
-                SinkIn<T, SRC, SNK, 1> in;
+            // cell x = j + R2 r of line l0 + l; kGroup entries' operands are in flight together,
+            // the first group's through the barrier (96 x 96 x 24, eight double-float right-hand
+            // sides: 451 -> 389 us with groups of three against one entry at a time)
+            constexpr int kGroup = 3;
+            SinkIn<T, SRC, SNK, kGroup> in;
+            int o[kGroup];
+            auto load = [&](int e0) {
+#pragma unroll
+                for (int k = 0; k < kGroup; k++) {
+                    const int e = e0 + k * NT, x = e / CT, ln = l0 + e % CT;
+                    o[k] = x < L.Nx && ln < NL ? line_entry<T>(L, NC, x, ln / 3, ln % 3) : -1;
+                }
                 in.load(R, o);
-                in.template store<NV>(R, o, &v, acc, out_ext);
+            };
+            load(threadIdx.x);
+            __syncthreads();
+            for (int e0 = threadIdx.x; e0 < L.Nx * CT; e0 += kGroup * NT) {
+                if (e0 != (int)threadIdx.x) load(e0);
+                cx<T> v[kGroup];
+#pragma unroll
+                for (int k = 0; k < kGroup; k++) {
+                    const int e = e0 + k * NT, x = e / CT;
+                    v[k] = o[k] >= 0 ? s[(x % R2) * TL::JS + (x / R2) * CT + e % CT] : czero<T>();
+                }
+                in.template store<NV>(R, o, v, acc, out_ext);
             }
         }
     } else {

@@ -66,6 +66,20 @@ struct __align__(16) dd2 {
     __host__ __device__ explicit dd2(float4 v) : x(v.x, v.y), y(v.z, v.w) {}
     __host__ __device__ double2 to_double2() const { return make_double2((double)x, (double)y); }
 };
+// dd(v) on the integer and FP32 pipes, for the loads of FP64 vectors (the gather of 80 x 80 x 20,
+// four right-hand sides: 60 -> 50 us; of 96 x 96 x 24, eight: 168 us either way.  The way back
+// made the scatter slower, 451 -> 476 us, and stays on the FP64 pipe).
+// hi is v rounded to its leading 24 bits (half added at bit 28), lo the signed low 29 bits,
+// both exact before lo's one rounding to 24 bits, as in the conversion above.
+// Values whose parts leave FP32's normal range take the conversion above.
+__device__ __forceinline__ dd dd_from_bits(double v) {
+    const unsigned hi = __double2hiint(v), lo = __double2loint(v), e = (hi >> 20) & 0x7ffu;
+    if (e - 949u > 200u) return v == 0.0 ? dd(0.f, 0.f) : dd(v);
+    const unsigned sg = hi & 0x80000000u, tl = lo + 0x10000000u, th = hi + (tl < lo ? 1u : 0u);
+    const unsigned h = (__funnelshift_l(tl, th, 3) - 0xC0000000u) & 0x7fffffffu;  // exponent bias 1023 -> 127
+    const int r = (int)(lo << 3) >> 3;
+    return dd(__uint_as_float(h | sg), __fmul_rn(__int2float_rn(r), __uint_as_float(((e - 948u) << 23) | sg)));
+}
 template <> struct cplx_t<dd> { typedef dd2 type; };
 template <typename T> constexpr bool is_dd = false;
 template <> constexpr bool is_dd<dd> = true;

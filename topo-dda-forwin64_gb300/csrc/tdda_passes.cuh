@@ -24,8 +24,12 @@ namespace dev {
 // writes the FP64 vectors (double2 in memory) and converts at the gather and
 // the scatter; the other precisions load and store their own type.
 template <typename T> __device__ __forceinline__ cx<T> ldv(const cx<T>* p, long long i) {
-    if constexpr (is_dd<T>) return dd2(reinterpret_cast<const double2*>(p)[i]);
-    else return p[i];
+    if constexpr (is_dd<T>) {
+        const double2 v = reinterpret_cast<const double2*>(p)[i];
+        return dd2(dd_from_bits(v.x), dd_from_bits(v.y));
+    } else {
+        return p[i];
+    }
 }
 template <typename T> __device__ __forceinline__ void stv(cx<T>* p, long long i, cx<T> v) {
     if constexpr (is_dd<T>) reinterpret_cast<double2*>(p)[i] = v.to_double2();
