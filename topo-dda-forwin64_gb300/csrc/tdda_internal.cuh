@@ -284,13 +284,12 @@ struct PeriodicImages {
     double Lm, Ln;   // periods, nm
 };
 
-// Green spectrum: LDR tensor on the full grid (the sum over the images when pi
-// is given, through the octant table oct of 6 Nx Ny Nz entries), 3-D forward
-// FFT, fold, scale.
+// Green spectrum: the LDR tensor (the sum over the images when pi is given) at
+// the octant of offsets, forward FFT along z, y, x, the octant k <= M / 2 of the
+// spectrum scaled.  Scratch: zk 6 Nx Ny Hz entries, oct 6 Nx Hy Hz.
 cudaError_t launch_green(const Geom& g, double K, double d, const double2* tw64x, const double2* tw64y,
-                         const double2* tw64z, double2* full6 /* 6*Mx*My*Mz scratch */, double2* green64,
-                         float2* green32, cudaStream_t stream, const Interaction& it,
-                         const PeriodicImages* pi = nullptr, double2* oct = nullptr);
+                         const double2* tw64z, double2* zk, double2* oct, double2* green64, float2* green32,
+                         cudaStream_t stream, const Interaction& it, const PeriodicImages* pi = nullptr);
 // the FCD Si/Ci tables (kSiCiN entries each)
 cudaError_t launch_sici_table(double* si, double* ci, cudaStream_t stream);
 

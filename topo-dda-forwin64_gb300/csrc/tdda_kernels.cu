@@ -258,52 +258,26 @@ __global__ void __launch_bounds__(kNT) k_green_periodic_octant(Geom g, double K,
     block_sum<12>(acc, sred);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int l = 0; l < 6; l++) oct[(long long)o * 6 + l] = make_double2(acc[2 * l], acc[2 * l + 1]);
+        for (int l = 0; l < 6; l++)
+            oct[((l * (long long)g.Ny + oy) * g.Nx + ox) * g.Nz + oz] = make_double2(acc[2 * l], acc[2 * l + 1]);
     }
 }
 
-// the full padded grid from the octant: xx, yy, zz even in every axis; xy odd
-// in x and y, xz in x and z, yz in y and z
 // The tensor at the octant of lattice offsets (0 <= o < N on each axis), one
-// thread per offset: every other offset differs only by the sign of the odd
-// components (xy odd in x and y, xz in x and z, yz in y and z), which
-// k_green_expand applies, so the FP64 tensor is evaluated Nx Ny Nz times
-// instead of once per grid point.
+// thread per offset, as six arrays [y][x][z]: every other offset differs only by
+// the sign of the odd components (xy odd in x and y, xz in x and z, yz in y and
+// z; xx, yy, zz even), so the FP64 tensor is evaluated Nx Ny Nz times instead of
+// once per grid point.
 __global__ void k_green_octant(Geom g, double K, double d, Interaction it, double2* __restrict__ oct) {
     const long long n = (long long)g.Nx * g.Ny * g.Nz;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
         const int oz = (int)(e % g.Nz);
-        const int oy = (int)((e / g.Nz) % g.Ny);
-        const int ox = (int)(e / ((long long)g.Nz * g.Ny));
+        const int ox = (int)((e / g.Nz) % g.Nx);
+        const int oy = (int)(e / ((long long)g.Nz * g.Nx));
         double2 t[6];
         interaction_tensor(it, K, d, d * ox, d * oy, d * oz, t);
 #pragma unroll
-        for (int l = 0; l < 6; l++) oct[e * 6 + l] = t[l];
-    }
-}
-__global__ void k_green_expand(Geom g, const double2* __restrict__ oct, double2* __restrict__ full6) {
-    const int Mx = g.px.M, My = g.py.M, Mz = g.pz.M;
-    const long long M = (long long)Mx * My * Mz;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < M; e += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(e % Mz);
-        const int j = (int)((e / Mz) % My);
-        const int i = (int)(e / ((long long)Mz * My));
-        int ox = i < g.Nx ? i : (i > Mx - g.Nx ? i - Mx : INT32_MIN);
-        int oy = j < g.Ny ? j : (j > My - g.Ny ? j - My : INT32_MIN);
-        int oz = k < g.Nz ? k : (k > Mz - g.Nz ? k - Mz : INT32_MIN);
-        double2 t[6];
-        if (ox != INT32_MIN && oy != INT32_MIN && oz != INT32_MIN) {
-            const double sx = ox < 0 ? -1.0 : 1.0, sy = oy < 0 ? -1.0 : 1.0, sz = oz < 0 ? -1.0 : 1.0;
-            const double2* src = oct + (((long long)abs(ox) * g.Ny + abs(oy)) * g.Nz + abs(oz)) * 6;
-            const double sg[6] = {1.0, sx * sy, sx * sz, 1.0, sy * sz, 1.0};
-#pragma unroll
-            for (int l = 0; l < 6; l++) t[l] = make_double2(sg[l] * src[l].x, sg[l] * src[l].y);
-        } else {
-#pragma unroll
-            for (int l = 0; l < 6; l++) t[l] = make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int l = 0; l < 6; l++) full6[l * M + e] = t[l];
+        for (int l = 0; l < 6; l++) oct[l * n + e] = t[l];
     }
 }
 
@@ -313,34 +287,10 @@ __global__ void k_sici_table(double* __restrict__ si, double* __restrict__ ci) {
         sici(kSiCiDis * (k + 1), &si[k], &ci[k]);
 }
 
-// fold the spectrum to the octant, scale by 1/M, write FP64 and FP32 copies
-__global__ void k_green_fold(Geom g, const double2* __restrict__ full6, double2* __restrict__ green64,
-                             float2* __restrict__ green32) {
-    const int Mx = g.px.M, My = g.py.M, Mz = g.pz.M;
-    const long long M = (long long)Mx * My * Mz;
-    const long long H = (long long)g.Hx * g.Hy * g.Hz;
-    const double inv = 1.0 / (double)M;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < H * 6; e += (long long)gridDim.x * blockDim.x) {
-        const int l = (int)(e % 6);
-        const long long q = e / 6;
-        const int fz = (int)(q % g.Hz);
-        const int fx = (int)((q / g.Hz) % g.Hx);
-        const int fy = (int)(q / ((long long)g.Hx * g.Hz));
-        const double2 v = full6[l * M + ((long long)fx * My + fy) * Mz + fz];
-        const double2 w = make_double2(v.x * inv, v.y * inv);
-        green64[fx * g.gs64.x + fy * g.gs64.y + fz * g.gs64.z + l * g.gs64.l] = w;
-        // FP32: planes of component pairs
-        green32[(fx * g.gs32.x + fy * g.gs32.y + fz * g.gs32.z + (l / 2) * g.gs32.l) * 2 + (l & 1)] =
-            make_float2((float)w.x, (float)w.y);
-    }
-}
-
 // ------------------------------------------------------- generic FFT passes
 // rows: nrows contiguous lines of length M
-// nout: outputs m >= nout are neither formed in the last stage nor stored (the
-// Green spectrum keeps only the octant k <= M / 2 of each axis)
 __global__ void __launch_bounds__(kNT) k_fft_rows(double2* __restrict__ data, long long nrows, AxisPlan p,
-                                                  const double2* __restrict__ tw, int sign, int nout) {
+                                                  const double2* __restrict__ tw, int sign) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int M = p.M;
     const int L = row_lines(p);
@@ -356,11 +306,11 @@ __global__ void __launch_bounds__(kNT) k_fft_rows(double2* __restrict__ data, lo
         s[line * MP + m] = data[(r0 + line) * M + m];
     }
     __syncthreads();
-    const double2* res = sign < 0 ? smem_fft<-1, double>(s, s2, L, MP, 1, p, stw, M, nout)
-                                  : smem_fft<+1, double>(s, s2, L, MP, 1, p, stw, M, nout);
+    const double2* res = sign < 0 ? smem_fft<-1, double>(s, s2, L, MP, 1, p, stw, M, M)
+                                  : smem_fft<+1, double>(s, s2, L, MP, 1, p, stw, M, M);
     for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
         const int line = e / M, m = e - (e / M) * M;
-        if (m < nout) data[(r0 + line) * M + m] = res[line * MP + m];
+        data[(r0 + line) * M + m] = res[line * MP + m];
     }
 }
 
@@ -368,7 +318,7 @@ __global__ void __launch_bounds__(kNT) k_fft_rows(double2* __restrict__ data, lo
 // contiguous; off(o) = (o / o1) * s1 + (o % o1) * s2
 __global__ void __launch_bounds__(kNT) k_fft_cols(double2* __restrict__ data, int nouter, int o1, long long s1,
                                                   long long s2, long long ms, int ninner, AxisPlan p,
-                                                  const double2* __restrict__ tw, int sign, int nout) {
+                                                  const double2* __restrict__ tw, int sign) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int M = p.M;
     const int ZT = col_tile(p);
@@ -385,11 +335,97 @@ __global__ void __launch_bounds__(kNT) k_fft_cols(double2* __restrict__ data, in
         s[e] = zl < zn ? base[m * ms + zl] : make_double2(0.0, 0.0);
     }
     __syncthreads();
-    const double2* res = sign < 0 ? smem_fft<-1, double>(s, sb2, ZT, 1, ZT, p, stw, M, nout)
-                                  : smem_fft<+1, double>(s, sb2, ZT, 1, ZT, p, stw, M, nout);
-    for (int e = threadIdx.x; e < nout * ZT; e += blockDim.x) {
+    const double2* res = sign < 0 ? smem_fft<-1, double>(s, sb2, ZT, 1, ZT, p, stw, M, M)
+                                  : smem_fft<+1, double>(s, sb2, ZT, 1, ZT, p, stw, M, M);
+    for (int e = threadIdx.x; e < M * ZT; e += blockDim.x) {
         const int m = e / ZT, zl = e - (e / ZT) * ZT;
         if (zl < zn) base[m * ms + zl] = res[e];
+    }
+}
+
+// ---------------------------------------------------------- Green spectrum
+// A line of the padded tensor is formed from the octant as it is loaded: entry m
+// is offset m, or M - m with the component's parity, or 0 between.  Transforming
+// along one axis keeps the parity along the others, so each pass transforms
+// octant lines only and keeps the outputs k <= M / 2: Nx Ny + Nx Hz + Hy Hz lines
+// of a component, against Mx My + Mx Hz + Hy Hz from a full grid (FP64
+// pipe; 96 x 96 x 24 box: 934 us with an expansion to the full grid and a fold
+// kernel, 391 us so; 40 x 40 x 12: 105 and 57).
+__device__ __forceinline__ double2 mirrored_entry(const double2* __restrict__ line, long long step, int m, int M, int N,
+                                                  bool odd) {
+    if (m < N) return line[m * step];
+    if (m <= M - N) return make_double2(0.0, 0.0);
+    const double2 v = line[(M - m) * step];
+    return odd ? make_double2(-v.x, -v.y) : v;
+}
+// z: rows [l][y][x] of N offsets -> the same rows of Hz outputs
+__global__ void __launch_bounds__(kNT) k_green_rows(const double2* __restrict__ in, double2* __restrict__ out,
+                                                    Geom g, const double2* __restrict__ tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const AxisPlan& p = g.pz;
+    const int M = p.M, H = g.Hz, N = g.Nz;
+    const int L = row_lines(p), MP = pad_odd(M);
+    double2* stw = reinterpret_cast<double2*>(smem_raw);
+    double2* s = stw + M;
+    double2* s2 = s + L * MP;
+    stage_tw<double>(stw, tw, M);
+    const long long per = (long long)g.Nx * g.Ny, r0 = (long long)blockIdx.x * L;
+    const int nl = (int)min((long long)L, 6 * per - r0);
+    for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
+        const int line = e / M, m = e - line * M, l = (int)((r0 + line) / per);
+        s[line * MP + m] = mirrored_entry(in + (r0 + line) * N, 1, m, M, N, l == 2 || l == 4);
+    }
+    __syncthreads();
+    const double2* res = smem_fft<-1, double>(s, s2, L, MP, 1, p, stw, M, H);
+    for (int e = threadIdx.x; e < nl * H; e += blockDim.x) {
+        const int line = e / H, m = e - line * H;
+        out[(r0 + line) * H + m] = res[line * MP + m];
+    }
+}
+// y: [l][y][x, kz] -> [l][x][kz, ky]; x: [l][x][kz, ky] -> the two spectra,
+// scaled by 1 / (Mx My Mz).  The pair (kz, ky) has the faster index of the
+// spectra's layout last (GreenStride), so the last stores are contiguous.
+template <bool X>
+__global__ void __launch_bounds__(kNT) k_green_cols(const double2* __restrict__ in, double2* __restrict__ out,
+                                                    float2* __restrict__ out32, Geom g,
+                                                    const double2* __restrict__ tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const AxisPlan& p = X ? g.px : g.py;
+    const int M = p.M, H = X ? g.Hx : g.Hy, N = X ? g.Nx : g.Ny, Hz = g.Hz, Hy = g.Hy;
+    const int ninner = X ? Hy * Hz : g.Nx * Hz;
+    const int ZT = col_tile(p), nt = (ninner + ZT - 1) / ZT;
+    const int l = blockIdx.x / nt, t0 = (blockIdx.x - l * nt) * ZT, zn = min(ZT, ninner - t0);
+    double2* stw = reinterpret_cast<double2*>(smem_raw);
+    double2* s = stw + M;
+    double2* s2 = s + M * ZT;
+    stage_tw<double>(stw, tw, M);
+    const double2* base = in + (long long)l * N * ninner + t0;
+    const bool odd = X ? l == 1 || l == 2 : l == 1 || l == 4, yfast = g.gs64.y == 1;
+    for (int e = threadIdx.x; e < M * ZT; e += blockDim.x) {
+        const int m = e / ZT, zl = e - m * ZT;
+        s[e] = zl < zn ? mirrored_entry(base + zl, ninner, m, M, N, odd) : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    const double2* res = smem_fft<-1, double>(s, s2, ZT, 1, ZT, p, stw, M, H);
+    const double inv = 1.0 / (double)((long long)g.px.M * g.py.M * g.pz.M);
+    for (int e = threadIdx.x; e < H * ZT; e += blockDim.x) {
+        int m, zl;
+        if (!X && yfast) zl = e / H, m = e - zl * H;
+        else m = e / ZT, zl = e - m * ZT;
+        if (zl >= zn) continue;
+        const double2 v = res[m * ZT + zl];
+        const int t = t0 + zl;
+        if constexpr (!X) {
+            const int x = t / Hz, kz = t - x * Hz;
+            out[((long long)l * g.Nx + x) * (Hy * Hz) + (yfast ? kz * Hy + m : m * Hz + kz)] = v;
+        } else {
+            const int ky = yfast ? t % Hy : t / Hz, kz = yfast ? t / Hy : t % Hz;
+            const double2 w = make_double2(v.x * inv, v.y * inv);
+            out[m * g.gs64.x + ky * g.gs64.y + kz * g.gs64.z + l * g.gs64.l] = w;
+            // FP32: planes of component pairs
+            out32[(m * g.gs32.x + ky * g.gs32.y + kz * g.gs32.z + (l / 2) * g.gs32.l) * 2 + (l & 1)] =
+                make_float2((float)w.x, (float)w.y);
+        }
     }
 }
 
@@ -665,6 +701,9 @@ cudaError_t configure_kernels() {
         e = cudaFuncSetAttribute((const void*)k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPassSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_fft_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPassSmem);
+    const void* green[] = {(const void*)k_green_rows, (const void*)k_green_cols<false>, (const void*)k_green_cols<true>};
+    for (const void* k : green)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPassSmem);
     return e;
 }
 
@@ -691,55 +730,37 @@ int max_blocks_per_rhs(const Geom& g) {
 // ------------------------------------------------------------------ launchers
 namespace {
 cudaError_t fft_rows(double2* data, long long nrows, const AxisPlan& p, const double2* tw, int sign,
-                     cudaStream_t stream, int nout = 0) {
+                     cudaStream_t stream) {
     const int L = row_lines(p);
-    k_fft_rows<<<(unsigned)((nrows + L - 1) / L), kNT, rowsmem(p), stream>>>(data, nrows, p, tw, sign,
-                                                                              nout > 0 ? nout : p.M);
+    k_fft_rows<<<(unsigned)((nrows + L - 1) / L), kNT, rowsmem(p), stream>>>(data, nrows, p, tw, sign);
     return cudaGetLastError();
 }
 cudaError_t fft_cols(double2* data, int nouter, int o1, long long s1, long long s2, long long ms, int ninner,
-                     const AxisPlan& p, const double2* tw, int sign, cudaStream_t stream, int nout = 0) {
+                     const AxisPlan& p, const double2* tw, int sign, cudaStream_t stream) {
     const int ZT = col_tile(p);
     const int nt = (ninner + ZT - 1) / ZT;
-    k_fft_cols<<<(unsigned)(nouter * nt), kNT, colsmem(p), stream>>>(data, nouter, o1, s1, s2, ms, ninner, p, tw,
-                                                                      sign, nout > 0 ? nout : p.M);
+    k_fft_cols<<<(unsigned)(nouter * nt), kNT, colsmem(p), stream>>>(data, nouter, o1, s1, s2, ms, ninner, p, tw, sign);
     return cudaGetLastError();
 }
 }  // namespace
 
 cudaError_t launch_green(const Geom& g, double K, double d, const double2* twx, const double2* twy, const double2* twz,
-                         double2* full6, double2* green64, float2* green32, cudaStream_t stream,
-                         const Interaction& it, const PeriodicImages* pi, double2* oct) {
-    const int Mx = g.px.M, My = g.py.M, Mz = g.pz.M;
-    const long long M = (long long)Mx * My * Mz;
-    cudaError_t err;
+                         double2* zk, double2* oct, double2* green64, float2* green32, cudaStream_t stream,
+                         const Interaction& it, const PeriodicImages* pi) {
     if (pi) {
         k_green_periodic_octant<<<g.Nx * g.Ny * g.Nz, kNT, 0, stream>>>(g, K, d, *pi, it, oct);
-        err = cudaGetLastError();
-        if (!err) {
-            k_green_expand<<<grid1d(M, kNT), kNT, 0, stream>>>(g, oct, full6);
-            err = cudaGetLastError();
-        }
     } else {
-        const long long n = (long long)g.Nx * g.Ny * g.Nz;
-        k_green_octant<<<grid1d(n, kNT), kNT, 0, stream>>>(g, K, d, it, oct);
-        err = cudaGetLastError();
-        if (!err) {
-            k_green_expand<<<grid1d(M, kNT), kNT, 0, stream>>>(g, oct, full6);
-            err = cudaGetLastError();
-        }
+        k_green_octant<<<grid1d((long long)g.Nx * g.Ny * g.Nz, 64), 64, 0, stream>>>(g, K, d, it, oct);
     }
-    // the six components form a (6 Mx, My, Mz) array for the z and y axes;
-    // the x axis runs over the outer pairs (component, y).  Only the octant
-    // k <= M / 2 of each axis is folded, so each axis forms only those outputs,
-    // and the later axes transform only the lines of the kept indices: the y
-    // pass the columns kz < Hz, the x pass the columns ky < Hy, kz < Hz.
-    if (!err) err = fft_rows(full6, 6LL * Mx * My, g.pz, twz, -1, stream, g.Hz);
-    if (!err) err = fft_cols(full6, 6 * Mx, 6 * Mx, 0, (long long)My * Mz, Mz, g.Hz, g.py, twy, -1, stream, g.Hy);
-    if (!err) err = fft_cols(full6, 6 * g.Hy, g.Hy, M, Mz, (long long)My * Mz, g.Hz, g.px, twx, -1, stream, g.Hx);
+    cudaError_t err = cudaGetLastError();
     if (err) return err;
-    const long long H6 = 6LL * g.Hx * g.Hy * g.Hz;
-    k_green_fold<<<grid1d(H6, kNT), kNT, 0, stream>>>(g, full6, green64, green32);
+    const long long rows = 6LL * g.Nx * g.Ny, L = row_lines(g.pz);
+    k_green_rows<<<(unsigned)((rows + L - 1) / L), kNT, rowsmem(g.pz), stream>>>(oct, zk, g, twz);
+    if ((err = cudaGetLastError())) return err;
+    const auto cols = [](const AxisPlan& p, int ninner) { return 6 * ((ninner + col_tile(p) - 1) / col_tile(p)); };
+    k_green_cols<false><<<cols(g.py, g.Nx * g.Hz), kNT, colsmem(g.py), stream>>>(zk, oct, nullptr, g, twy);
+    if ((err = cudaGetLastError())) return err;
+    k_green_cols<true><<<cols(g.px, g.Hy * g.Hz), kNT, colsmem(g.px), stream>>>(oct, green64, green32, g, twx);
     return cudaGetLastError();
 }
 
