@@ -570,13 +570,14 @@ template <typename T> int group_count(const tdda_core* c, int n) {
 // six pass events) is recorded for an ungrouped product only.
 template <typename T>
 cudaError_t aprod(tdda_core* c, int src, int snk, int n, const RhsVecs<T>* rhs, cudaEvent_t* ev = nullptr,
-                  int slot = 0) {
+                  int slot = 0, cudaStream_t stream = nullptr, long long grid_at = 0) {
     const int gs = group_size<T>(c, n);
     for (int g0 = 0; g0 < n; g0 += gs) {
         count_launches(product_kernels<T>(c));
         const cudaError_t e = tdda::launch_aproduct<T>(
             c->g, src, snk, std::min(gs, n - g0), rhs + g0, Prec<T>::green(c), Prec<T>::tw(c, 0), Prec<T>::tw(c, 1),
-            Prec<T>::tw(c, 2), c->cellmap, Prec<T>::grid(c), c->stream, gs == n ? ev : nullptr, slot);
+            Prec<T>::tw(c, 2), c->cellmap, Prec<T>::grid(c) + grid_at, stream ? stream : c->stream,
+            gs == n ? ev : nullptr, slot);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -592,17 +593,21 @@ cudaError_t aprod(tdda_core* c, int src, int snk, int n, const RhsVecs<T>* rhs, 
 // them in the state slots of the step's parity `slot`.
 template <typename T> constexpr bool kDeferred = sizeof(T) == 4;
 
+template <typename T> int solve_branches(const tdda_core* c, int n);
 template <typename T> int step_kernels(const tdda_core* c, int n) {
-    return 2 * product_kernels<T>(c) * group_count<T>(c, n) + (kDeferred<T> ? 0 : 1);
+    return 2 * product_kernels<T>(c) * group_count<T>(c, n) * solve_branches<T>(c, n) + (kDeferred<T> ? 0 : 1);
 }
 
-template <typename T> cudaError_t enqueue_iteration(tdda_core* c, int n, int slot) {
-    const RhsVecs<T>* rhs = Prec<T>::rhs(c);
+// One step of the n right-hand sides from `first` on, on `stream`.
+template <typename T> cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStream_t stream) {
+    const RhsVecs<T>* rhs = Prec<T>::rhs(c) + first;
+    const long long at = first * grid_entries(c->g);
     cudaError_t e;
     if constexpr (kDeferred<T>) {
         // update, p, Ap
-        if ((e = aprod<T>(c, tdda::SRC_PUPD_DEF, tdda::SNK_AP, n, rhs, nullptr, slot))) return e;
-        return aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT_DEF, n, rhs, nullptr, slot);  // alpha, t, At
+        if ((e = aprod<T>(c, tdda::SRC_PUPD_DEF, tdda::SNK_AP, n, rhs, nullptr, slot, stream, at))) return e;
+        // alpha, t, At
+        return aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT_DEF, n, rhs, nullptr, slot, stream, at);
     } else {
         if ((e = aprod<T>(c, tdda::SRC_PUPD, tdda::SNK_AP, n, rhs))) return e;  // p, Ap, alpha
         if ((e = aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT, n, rhs))) return e;  // t, At, zeta
@@ -611,15 +616,80 @@ template <typename T> cudaError_t enqueue_iteration(tdda_core* c, int n, int slo
     }
 }
 
+// The FP32 steps of a batch run as parallel branches of the graph, each with its
+// share of the right-hand sides, which are independent until the chunk's end:
+// where one branch's kernel runs out of blocks, another's take the SMs.  The
+// plane kernel keeps one block an SM, so a batch of 4.2 waves otherwise pays for
+// five (80 x 80 x 20, four right-hand sides: 186 -> 172 us a step; 45 x 33 x 19,
+// two: 47 -> 43; 128 x 128 x 32, two: 507 -> 469; priorities among the branches
+// change nothing).  Two branches, but
+//  - one where all planes fit one wave (13 x 100 x 9, four: 37.5 us, in two 38.1);
+//  - four (of one right-hand side or more) where two right-hand sides are about a
+//    wave, which halves would overshoot, up to five waves (37 x 51 x 13, four:
+//    71 us, in two 74, in four 65; 40 x 40 x 12, eight: 78, 79 and 76, but
+//    twelve, 6.3 waves: 106, 101 and 108);
+//  - three for three (80 x 80 x 20: 141 us, in two 134, in three 131);
+//  - one for plane blocks that take nearly all of an SM's shared memory where the
+//    last wave is nearly full or the launch long, whose tails are short beside what
+//    the branches cost (41 x 90 x 23, three, 1.9 waves: 113 us, in three 116;
+//    96 x 96 x 24: six 449 us, in two 453; eight 600 and 605; twelve 870 and 898).
+constexpr int kMaxBranches = 4;
+template <typename T> int solve_branches(const tdda_core* c, int n) {
+    const Geom& g = c->g;
+    const tdda::ProductForm form = tdda::product_form(g, true);
+    if (!kDeferred<T> || n < 2 || group_count<T>(c, n) > 1 || form < tdda::FORM_AXES) return 1;
+    const long long planes = (long long)n * g.px.M, sms = g.sms > 0 ? g.sms : 152;
+    const long long plane_bytes = 3LL * sizeof(float2) * g.py.M * g.pz.M;
+    if (planes <= sms) return 1;
+    if (form == tdda::FORM_PLANE && plane_bytes > 200 * 1024 && (planes > 7 * sms || 20 * (planes % sms) > 17 * sms))
+        return 1;
+    if (20LL * g.px.M <= 11 * sms && planes <= 5 * sms) return std::min(n, kMaxBranches);
+    return n == 3 ? 3 : 2;
+}
+struct Branches {
+    int count = 1;
+    cudaStream_t s[kMaxBranches] = {};
+    cudaEvent_t fork = nullptr, join[kMaxBranches] = {};
+    cudaError_t create(int n, cudaStream_t own) {
+        count = n;
+        s[0] = own;
+        if (n < 2) return cudaSuccess;
+        cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        for (int i = 1; i < n && e == cudaSuccess; i++) {
+            e = cudaStreamCreateWithFlags(&s[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming);
+        }
+        return e;
+    }
+    ~Branches() {
+        if (fork) cudaEventDestroy(fork);
+        for (int i = 1; i < kMaxBranches; i++) {
+            if (join[i]) cudaEventDestroy(join[i]);
+            if (s[i]) cudaStreamDestroy(s[i]);
+        }
+    }
+};
+
 // kChunk steps (parities 0, 1, 0, 1 ...); FP32 ends the chunk with the step
 // end for the next step (parity 0) and the condition of the device-side loop
 template <typename T>
-cudaError_t enqueue_chunk(tdda_core* c, int n, cudaGraphConditionalHandle loop, bool in_loop) {
-    for (int k = 0; k < kChunk; k++) {
-        cudaError_t e = enqueue_iteration<T>(c, n, k & 1);
-        if (e != cudaSuccess) return e;
+cudaError_t enqueue_chunk(tdda_core* c, int n, const Branches& br, cudaGraphConditionalHandle loop, bool in_loop) {
+    cudaError_t e = cudaSuccess;
+    if (br.count > 1) e = cudaEventRecord(br.fork, c->stream);
+    for (int b = 0; b < br.count; b++) {
+        const int first = (int)((long long)n * b / br.count), end = (int)((long long)n * (b + 1) / br.count);
+        if (e == cudaSuccess && b > 0) e = cudaStreamWaitEvent(br.s[b], br.fork, 0);
+        for (int k = 0; k < kChunk && e == cudaSuccess; k++)
+            e = enqueue_iteration<T>(c, first, end - first, k & 1, br.s[b]);
+        if (e == cudaSuccess && b > 0) e = cudaEventRecord(br.join[b], br.s[b]);
     }
-    if constexpr (kDeferred<T>) return tdda::launch_chunk_end(c->g, n, Prec<T>::rhs(c), 0, loop, in_loop, c->stream);
+    for (int b = 1; b < br.count && e == cudaSuccess; b++) e = cudaStreamWaitEvent(c->stream, br.join[b], 0);
+    if (e != cudaSuccess) return e;
+    if constexpr (kDeferred<T>) {
+        Geom g = c->g;
+        if (br.count > 1) g.early = 0;  // it follows several kernels
+        return tdda::launch_chunk_end(g, n, Prec<T>::rhs(c), 0, loop, in_loop, c->stream);
+    }
     return cudaSuccess;
 }
 template <typename T> int chunk_kernels(const tdda_core* c, int n) {
@@ -635,6 +705,8 @@ template <typename T> tdda_status get_iteration_graph(tdda_core* c, int n, cudaG
     if (!ex) {
         cudaGraph_t gr = nullptr;
         cudaError_t e = cudaSuccess, e2 = cudaSuccess;
+        Branches br;
+        TDDA_CK(br.create(solve_branches<T>(c, n), c->stream));
         if (kDeferred<T> && c->device_loop) {
             TDDA_CK(cudaGraphCreate(&gr, 0));
             cudaGraphConditionalHandle loop = 0;
@@ -653,14 +725,14 @@ template <typename T> tdda_status get_iteration_graph(tdda_core* c, int n, cudaG
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             TDDA_CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             t_capturing = true;
-            e = enqueue_chunk<T>(c, n, loop, true);
+            e = enqueue_chunk<T>(c, n, br, loop, true);
             t_capturing = false;
             cudaGraph_t captured = nullptr;
             e2 = cudaStreamEndCapture(c->stream, &captured);
         } else {
             TDDA_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             t_capturing = true;
-            e = enqueue_chunk<T>(c, n, 0, false);
+            e = enqueue_chunk<T>(c, n, br, 0, false);
             t_capturing = false;
             e2 = cudaStreamEndCapture(c->stream, &gr);
         }
