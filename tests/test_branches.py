@@ -36,3 +36,30 @@ def test_batch_equals_alone(box, n, branches, loop, monkeypatch):
     for m in ms:
         m.close()
     core.close()
+
+
+@pytest.mark.gpu
+def test_cross_lattice_models_of_one_core_equal_alone():
+    """The residuals of a cross-lattice batch run together where the cores differ and in turn where
+    models share one: two models of one core beside one of another, bit by bit as alone."""
+    if tdda.device_count() < 1:
+        pytest.skip("no CUDA device")
+    rng = np.random.Generator(np.random.PCG64(5))
+    inc = lattice.config(3).incidences
+    cores, ms = [], []
+    for box, count in (((20, 20, 10), 2), ((18, 19, 9), 1)):
+        R = lattice.bulk(*box)
+        cores.append(tdda.AProductCore(*box, R, 10.0, 520.0, np.array([1.0, 4.0 + 0.1j])))
+        for _ in range(count):
+            i = inc[len(ms)]
+            ms.append(tdda.DDAModel(cores[-1], i.nK, i.E0, i.nE0, np.repeat(rng.random(R.size // 3), 3)))
+    tdda.solve_multi(ms, 400, 1e-9)
+    together = [m.get_P() for m in ms]
+    for m, P in zip(ms, together):
+        m.InitializeP()
+        m.solve_mixed(400, 1e-9)
+        assert np.array_equal(m.get_P(), P)
+    for m in ms:
+        m.close()
+    for c in cores:
+        c.close()
