@@ -191,6 +191,7 @@ struct tdda_core_s {
     int* cellmap = nullptr;
     int* Rdev = nullptr;  // 3N lattice indices
     double2* green64 = nullptr;
+    double2* table = nullptr;  // the octant of the tensor, where plain FP64 products are summed directly
     // FP32 inner solve as a device-side loop (conditional graph node); TDDA_DEVICE_LOOP=0 in the
     // environment makes the host launch each chunk instead (profilers see the kernels of a
     // host-launched graph, not those of a device-side loop's body)
@@ -553,6 +554,16 @@ void grid_layout(Geom* g) {
         g->gs32 = {3 * Hz, 3 * Hz * Hx, 1, Hz};
         g->gs64 = {6 * Hz, 6 * Hz * Hx, 6, 1};
     }
+}
+// Plain FP64 products are summed directly up to kDirectDipoles, where the pairs
+// cost what the transforms do (direct and FFT: 512 dipoles of 8 x 8 x 8 36 and 44
+// us a call, 600 of 10 x 10 x 6 42 and 41; boxes without compiled axis kernels
+// cross near 900), and where the table of the tensor stays small beside L2.
+// TDDA_DIRECT=0 in the environment keeps the transforms for all.
+constexpr int kDirectDipoles = 512;
+bool direct_products(const Geom& g) {
+    const char* v = std::getenv("TDDA_DIRECT");
+    return !(v && v[0] == '0') && g.N <= kDirectDipoles && (long long)g.Nx * g.Ny * g.Nz <= 16 * kDirectDipoles;
 }
 // entries of the work grid of one right-hand side, whichever form runs
 long long grid_entries(const Geom& g) { return std::max(g.sb, g.vb); }
@@ -1326,7 +1337,7 @@ double core_bytes(int Nx, int Ny, int Nz, int N, int max_rhs) {
            + 6 * H * (16 + 8 + 16)                     // Green spectra (FP64, FP32, double-float)
            + grid * (16 + 8)                           // FP64 and FP32 grids
            + n3 * 2 * (16 + 8)                         // product staging
-           + 6 * Mx * My * Mz * 16                     // full Green grid while the core is built
+           + 6 * Mx * My * Mz * 16                     // scratch while the core is built (at most), direct table
            + 1e6;                                      // reduction partials, states, twiddles
 }
 
@@ -1808,6 +1819,7 @@ tdda_status core_create(const tdda_core_desc* desc, const tdda::PeriodicImages* 
     TDDA_CORE_TRY(dalloc_c(c, &c->Rdev, 3 * (size_t)g.N));
     TDDA_CORE_TRY(dalloc_c(c, &c->green64, (size_t)H6));
     TDDA_CORE_TRY(dalloc_c(c, &c->green32, (size_t)H6));
+    if (direct_products(g)) TDDA_CORE_TRY(dalloc_c(c, &c->table, 6 * (size_t)g.Nx * g.Ny * g.Nz));
     for (int a = 0; a < 3; a++) {
         TDDA_CORE_TRY(dalloc_c(c, &c->tw64[a], (size_t)plans[a]->M));
         TDDA_CORE_TRY(dalloc_c(c, &c->tw32[a], (size_t)plans[a]->M));
@@ -1860,7 +1872,7 @@ tdda_status core_create(const tdda_core_desc* desc, const tdda::PeriodicImages* 
     if (ge == cudaSuccess) {
         count_launches(4);
         ge = tdda::launch_green(g, c->K, c->d, c->tw64[0], c->tw64[1], c->tw64[2], zk, oct, c->green64, c->green32,
-                                c->stream, c->inter, pi);
+                                c->stream, c->inter, pi, c->table);
         const cudaError_t fe = cudaFreeAsync(oct, c->stream);
         if (ge == cudaSuccess) ge = fe;
     }
@@ -1954,20 +1966,25 @@ tdda_status tdda_aproduct(tdda_core* c, int precision, const double* b, double* 
     TDDA_TRY(set_device(c->device));
     const size_t n3 = 3 * (size_t)c->N;
     const bool fp64 = precision == TDDA_FP64;
-    if (tdda::product_form(c->g, !fp64) >= tdda::FORM_AXES) {
+    if ((fp64 && c->table) || tdda::product_form(c->g, !fp64) >= tdda::FORM_AXES) {
         // the x kernels read and write FP64 vectors themselves: a device caller's in
         // place where a kernel may touch them, else the core's staging vectors
         const double2* in = reinterpret_cast<const double2*>(b);
         double2* out = reinterpret_cast<double2*>(y);
         const bool own_in = mem == TDDA_MEM_DEVICE && kernel_may_use(b, c->device);
-        const bool own_out = mem == TDDA_MEM_DEVICE && kernel_may_use(y, c->device);
+        // the transforms read all of b before they write y; the direct sums do not
+        const uintptr_t ba = (uintptr_t)b, ya = (uintptr_t)y, bytes = sizeof(double2) * n3;
+        const bool apart = !(fp64 && c->table) || ba + bytes <= ya || ya + bytes <= ba;
+        const bool own_out = mem == TDDA_MEM_DEVICE && apart && kernel_may_use(y, c->device);
         if (!own_in) {
             TDDA_CK(cudaMemcpyAsync(c->vin64, b, sizeof(double2) * n3, kind_in(mem), c->stream));
             in = c->vin64;
         }
         if (!own_out) out = c->vout64;
-        count_launches(fp64 ? product_kernels<double>(c) : product_kernels<float>(c));
-        if (fp64) {
+        count_launches(fp64 && c->table ? 1 : fp64 ? product_kernels<double>(c) : product_kernels<float>(c));
+        if (fp64 && c->table) {
+            TDDA_CK(tdda::launch_direct(c->g, c->Rdev, c->table, in, out, c->stream));
+        } else if (fp64) {
             TDDA_CK(tdda::launch_aproduct_ext<double>(c->g, c->rhs64 + c->max_rhs, in, out, c->green64, c->tw64[0],
                                                       c->tw64[1], c->tw64[2], c->cellmap, c->grid64, c->stream));
         } else {

@@ -286,10 +286,15 @@ struct PeriodicImages {
 
 // Green spectrum: the LDR tensor (the sum over the images when pi is given) at
 // the octant of offsets, forward FFT along z, y, x, the octant k <= M / 2 of the
-// spectrum scaled.  Scratch: zk 6 Nx Ny Hz entries, oct 6 Nx Hy Hz.
+// spectrum scaled.  Scratch: zk 6 Nx Ny Hz entries, oct 6 Nx Hy Hz.  The octant
+// of the tensor stays in `table` (6 Nx Ny Nz entries) where one is given.
 cudaError_t launch_green(const Geom& g, double K, double d, const double2* tw64x, const double2* tw64y,
                          const double2* tw64z, double2* zk, double2* oct, double2* green64, float2* green32,
-                         cudaStream_t stream, const Interaction& it, const PeriodicImages* pi = nullptr);
+                         cudaStream_t stream, const Interaction& it, const PeriodicImages* pi = nullptr,
+                         double2* table = nullptr);
+// A_offdiag b by direct summation from the octant of the tensor (FP64, AoS vectors)
+cudaError_t launch_direct(const Geom& g, const int* R, const double2* table, const double2* in, double2* out,
+                          cudaStream_t stream);
 // the FCD Si/Ci tables (kSiCiN entries each)
 cudaError_t launch_sici_table(double* si, double* ci, cudaStream_t stream);
 

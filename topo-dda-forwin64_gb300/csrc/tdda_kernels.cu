@@ -429,6 +429,79 @@ __global__ void __launch_bounds__(kNT) k_green_cols(const double2* __restrict__ 
     }
 }
 
+// ------------------------------------------------------- direct products
+// y_i = sum_j G(r_i - r_j) b_j for lattices of few dipoles, from the octant of
+// the tensor [component][y][x][z]: five dependent FFT kernels of a few blocks
+// cost more than the N^2 pairs (call on device vectors, 8 x 7 x 5 box of 196: 64
+// -> 21 us; 8 x 8 x 8: 44 -> 36).  Bound by the FP64 pipe, 36 multiply-adds a pair.
+// A block sums two dipoles (more blocks than SMs from 300 dipoles on), its lanes
+// 16 neighbours at once and its warps interleaved neighbours (of 2, 4 and 8 warps:
+// 24, 21 and 20 us at 196 dipoles, 34, 30 and 31 at 384); each step of the
+// lane reduction halves the six sums a lane holds, so a warp adds 7 times, not 24.
+constexpr int kDirectWarps = 4;
+__global__ void __launch_bounds__(32 * kDirectWarps) k_direct(int N, const int* __restrict__ R, int Nx, int Ny, int Nz,
+                                                              const double2* __restrict__ oct,
+                                                              const double2* __restrict__ b,
+                                                              double* __restrict__ y) {
+    __shared__ double part[kDirectWarps][2][6];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
+    const int i = 2 * blockIdx.x + half, ic = min(i, N - 1);
+    const int xi = R[3 * ic], yi = R[3 * ic + 1], zi = R[3 * ic + 2];
+    const int ncomp = Nx * Ny * Nz;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int j = warp * 16 + (lane & 15); j < N; j += 16 * kDirectWarps) {
+        const int dx = xi - R[3 * j], dy = yi - R[3 * j + 1], dz = zi - R[3 * j + 2];
+        const double2* g = oct + ((abs(dy) * Nx + abs(dx)) * Nz + abs(dz));
+        double2 a[6];
+#pragma unroll
+        for (int l = 0; l < 6; l++) a[l] = __ldg(g + l * ncomp);
+        const double2 b0 = b[3 * j], b1 = b[3 * j + 1], b2 = b[3 * j + 2];
+        if ((dx ^ dy) < 0 && dx && dy) a[1] = make_double2(-a[1].x, -a[1].y);  // odd in x and y
+        if ((dx ^ dz) < 0 && dx && dz) a[2] = make_double2(-a[2].x, -a[2].y);  // odd in x and z
+        if ((dy ^ dz) < 0 && dy && dz) a[4] = make_double2(-a[4].x, -a[4].y);  // odd in y and z
+        const double2 row[3][3] = {{a[0], a[1], a[2]}, {a[1], a[3], a[4]}, {a[2], a[4], a[5]}};
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const double2 bb[3] = {b0, b1, b2};
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                v[2 * r] = fma(row[r][q].x, bb[q].x, v[2 * r]);
+                v[2 * r + 1] = fma(row[r][q].x, bb[q].y, v[2 * r + 1]);
+                v[2 * r] = fma(-row[r][q].y, bb[q].y, v[2 * r]);
+                v[2 * r + 1] = fma(row[r][q].y, bb[q].x, v[2 * r + 1]);
+            }
+        }
+    }
+    const unsigned all = 0xffffffffu;
+    const bool h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+    double p[4], q[2];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {  // lanes with bit 3 go on with the values 3 .. 5
+        const double got = __shfl_xor_sync(all, h8 ? v[k] : v[k + 3], 8);
+        p[k] = (h8 ? v[k + 3] : v[k]) + got;
+    }
+    p[3] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double got = __shfl_xor_sync(all, h4 ? p[k] : p[k + 2], 4);
+        q[k] = (h4 ? p[k + 2] : p[k]) + got;
+    }
+    const double got = __shfl_xor_sync(all, h2 ? q[0] : q[1], 2);
+    double t = (h2 ? q[1] : q[0]) + got;
+    t += __shfl_xor_sync(all, t, 1);
+    const int k = 2 * (h4 ? 1 : 0) + (h2 ? 1 : 0);  // value of this lane among its three
+    if (!(lane & 1) && k < 3) part[warp][half][3 * (h8 ? 1 : 0) + k] = t;
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        const int h = threadIdx.x / 6, e = threadIdx.x % 6, o = 2 * blockIdx.x + h;
+        double sum = 0.0;
+#pragma unroll
+        for (int w = 0; w < kDirectWarps; w++) sum += part[w][h][e];
+        if (o < N) y[6 * (long long)o + e] = sum;
+    }
+}
+
 // ------------------------------------------------------------ polarisability
 __device__ __forceinline__ double2 dadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 dscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
@@ -746,21 +819,29 @@ cudaError_t fft_cols(double2* data, int nouter, int o1, long long s1, long long 
 
 cudaError_t launch_green(const Geom& g, double K, double d, const double2* twx, const double2* twy, const double2* twz,
                          double2* zk, double2* oct, double2* green64, float2* green32, cudaStream_t stream,
-                         const Interaction& it, const PeriodicImages* pi) {
+                         const Interaction& it, const PeriodicImages* pi, double2* table) {
+    double2* at = table ? table : oct;
     if (pi) {
-        k_green_periodic_octant<<<g.Nx * g.Ny * g.Nz, kNT, 0, stream>>>(g, K, d, *pi, it, oct);
+        k_green_periodic_octant<<<g.Nx * g.Ny * g.Nz, kNT, 0, stream>>>(g, K, d, *pi, it, at);
     } else {
-        k_green_octant<<<grid1d((long long)g.Nx * g.Ny * g.Nz, 64), 64, 0, stream>>>(g, K, d, it, oct);
+        k_green_octant<<<grid1d((long long)g.Nx * g.Ny * g.Nz, 64), 64, 0, stream>>>(g, K, d, it, at);
     }
     cudaError_t err = cudaGetLastError();
     if (err) return err;
     const long long rows = 6LL * g.Nx * g.Ny, L = row_lines(g.pz);
-    k_green_rows<<<(unsigned)((rows + L - 1) / L), kNT, rowsmem(g.pz), stream>>>(oct, zk, g, twz);
+    k_green_rows<<<(unsigned)((rows + L - 1) / L), kNT, rowsmem(g.pz), stream>>>(at, zk, g, twz);
     if ((err = cudaGetLastError())) return err;
     const auto cols = [](const AxisPlan& p, int ninner) { return 6 * ((ninner + col_tile(p) - 1) / col_tile(p)); };
     k_green_cols<false><<<cols(g.py, g.Nx * g.Hz), kNT, colsmem(g.py), stream>>>(zk, oct, nullptr, g, twy);
     if ((err = cudaGetLastError())) return err;
     k_green_cols<true><<<cols(g.px, g.Hy * g.Hz), kNT, colsmem(g.px), stream>>>(oct, green64, green32, g, twx);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_direct(const Geom& g, const int* R, const double2* table, const double2* in, double2* out,
+                          cudaStream_t stream) {
+    k_direct<<<(g.N + 1) / 2, 32 * kDirectWarps, 0, stream>>>(g.N, R, g.Nx, g.Ny, g.Nz, table, in,
+                                                              reinterpret_cast<double*>(out));
     return cudaGetLastError();
 }
 
