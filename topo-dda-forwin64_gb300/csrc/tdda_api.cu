@@ -555,15 +555,16 @@ void grid_layout(Geom* g) {
         g->gs64 = {6 * Hz, 6 * Hz * Hx, 6, 1};
     }
 }
-// Plain FP64 products are summed directly up to kDirectDipoles, where the pairs
-// cost what the transforms do (direct and FFT: 512 dipoles of 8 x 8 x 8 36 and 44
-// us a call, 600 of 10 x 10 x 6 42 and 41; boxes without compiled axis kernels
-// cross near 900), and where the table of the tensor stays small beside L2.
+// Plain FP64 products are summed directly up to the number of dipoles where the
+// pairs cost what the transforms do (direct and FFT, us a call on device vectors:
+// 512 dipoles of 8 x 8 x 8 36 and 44, 600 of 10 x 10 x 6 42 and 41; on grids
+// without compiled axis kernels 320 of 20 x 4 x 4 27 and 81, 800 of 40 x 4 x 5 67
+// and 87), and where the table of the tensor stays small beside L2.
 // TDDA_DIRECT=0 in the environment keeps the transforms for all.
-constexpr int kDirectDipoles = 512;
 bool direct_products(const Geom& g) {
     const char* v = std::getenv("TDDA_DIRECT");
-    return !(v && v[0] == '0') && g.N <= kDirectDipoles && (long long)g.Nx * g.Ny * g.Nz <= 16 * kDirectDipoles;
+    const int limit = tdda::product_form(g, false) >= tdda::FORM_AXES ? 512 : 800;
+    return !(v && v[0] == '0') && g.N <= limit && (long long)g.Nx * g.Ny * g.Nz <= 8192;
 }
 // entries of the work grid of one right-hand side, whichever form runs
 long long grid_entries(const Geom& g) { return std::max(g.sb, g.vb); }
