@@ -748,6 +748,18 @@ template <typename T> constexpr bool kZFused = sizeof(T) == 4;
 template <typename T, int M, int RT> __host__ __device__ constexpr int zprod_threads() {
     return !kZFused<T> ? 128 : round32(RT * AxisZ<M>::R1) < 64 ? 64 : round32(RT * AxisZ<M>::R1);
 }
+// Rows of a full tile, points the FP32 spectrum's loads run ahead, and the threads
+// an SM has to hold (registers): what bounds the FP32 kernel is its loads' latency,
+// so the long lengths take smaller tiles, more blocks and loads further ahead
+// (steps of 110 x 100 x 24, z length 48: 168 us with 32 rows, 1 ahead and no
+// bound, 147 so; 80 x 100 x 28, 56: 139 and 119; 128 x 128 x 32, 64: 246 and 240,
+// where the bound costs 3 us; 60 x 128 x 20, 40: 91 and 83 with the bound alone,
+// 89 with the small tile).  The lengths below 40 lose with any of the three.
+template <typename T, int M> __host__ __device__ constexpr int zprod_wide() { return kZFused<T> && M < 48 ? 32 : 16; }
+template <int M, int RT> __host__ __device__ constexpr int zprod_ahead() { return M < 48 || RT < 16 ? 1 : 3; }
+template <typename T, int M, int RT> __host__ __device__ constexpr int zprod_minb() {  // 0: unspecified (1 lets the compiler take more registers: 128 x 128 x 32 288 us)
+    return kZFused<T> && M >= 40 && M < 64 && RT >= 16 ? 640 / zprod_threads<T, M, RT>() : 0;
+}
 // RT rows (kx, ky) of three components: row pitch odd, so that consecutive rows
 // start in different banks
 template <typename T, int M, int RT> struct ZTile {
@@ -755,10 +767,9 @@ template <typename T, int M, int RT> struct ZTile {
     static constexpr size_t smem = sizeof(cx<T>) * (size_t)(M + 3 * RT * ZP);
 };
 template <typename T, int M, int RT>
-__global__ void __launch_bounds__(zprod_threads<T, M, RT>()) k_zprod(Geom g, const RhsVecs<T>* __restrict__ rhs,
-                                                                     const cx<T>* __restrict__ green,
-                                                                     const cx<T>* __restrict__ twz,
-                                                                     cx<T>* __restrict__ grid) {
+__global__ void __launch_bounds__(zprod_threads<T, M, RT>(), zprod_minb<T, M, RT>())
+    k_zprod(Geom g, const RhsVecs<T>* __restrict__ rhs, const cx<T>* __restrict__ green, const cx<T>* __restrict__ twz,
+            cx<T>* __restrict__ grid) {
     using A = AxisZ<M>;
     constexpr int R1 = A::R1, R2 = A::R2, RH = A::RH, ZP = ZTile<T, M, RT>::ZP, NT = zprod_threads<T, M, RT>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -811,7 +822,7 @@ __global__ void __launch_bounds__(zprod_threads<T, M, RT>()) k_zprod(Geom g, con
             int kx, ky;
             row_k(row, kx, ky);
             if (kx >= Mx) continue;
-            SpectralRow<T, R1, R2, M, 1> sp(GreenRow<T>(green, g, fold(kx, Mx), fold(ky, My)), j);
+            SpectralRow<T, R1, R2, M, zprod_ahead<M, RT>()> sp(GreenRow<T>(green, g, fold(kx, Mx), fold(ky, My)), j);
             cx<T> X[3][R2];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -1201,8 +1212,8 @@ template <typename T, int M> struct ZprodLaunch {
         return launch_axis(a, k_zprod<T, M, RT>, grid, zprod_threads<T, M, RT>(), ZTile<T, M, RT>::smem, a.rhs, a.green,
                            a.twz, a.grid);
     }
-    // rows a block: 32 (FP32) or 16 where that leaves every SM several blocks, else 8
-    static constexpr int kWide = kZFused<T> ? 32 : 16;
+    // rows a block: the full tile where that leaves every SM several blocks, else 8
+    static constexpr int kWide = zprod_wide<T, M>();
     static cudaError_t run(const PassArgs<T>& a) {
         const long long rows = (long long)a.g.px.M * a.g.py.M * a.nrhs;
         return rows >= kWide * (kZFused<T> ? 4LL : 2LL) * 152 ? run1<kWide>(a) : run1<8>(a);
