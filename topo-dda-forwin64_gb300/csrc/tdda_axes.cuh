@@ -422,9 +422,11 @@ __global__ void __launch_bounds__(axis_threads<M, CT>(), axis_minb<M, CT>()) k_x
 // stage holds the cells x = j + R2 r of one line and scatters them; the sink's
 // operands do not depend on the transform, and their loads are issued before the
 // barrier.  FP64 and double-float: the cells go back to shared memory (in place)
-// and all threads of the block share them.
+// and all threads of the block share them.  The double-float kernel waits for
+// memory: registers for 768 threads an SM instead of 512 (96 x 96 x 24, four
+// right-hand sides: 213 -> 170 us; 640: 184; 80 x 80 x 20, two: 63 -> 62).
 template <typename T, int SRC, int SNK, int M, int CT>
-__global__ void __launch_bounds__(sink_threads<T, M, CT>()) k_xinv(Geom g, const RhsVecs<T>* __restrict__ rhs,
+__global__ void __launch_bounds__(sink_threads<T, M, CT>(), is_dd<T> ? 768 / sink_threads<T, M, CT>() : 0) k_xinv(Geom g, const RhsVecs<T>* __restrict__ rhs,
                                                                   const cx<T>* __restrict__ twx,
                                                                   const int* __restrict__ cellmap,
                                                                   const cx<T>* __restrict__ grid, int pitch_rows,
