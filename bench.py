@@ -165,6 +165,22 @@ def pass_bytes(grid, Nx, Ny, Nz, N, s, fused=False):
     return [zf * s, yf * s, xp * s, yf * s, zf * s]
 
 
+def slot_bytes(names, grid, Nx, Ny, Nz, N, s):
+    """Algorithmic bytes of each profile slot of one A-product for one right-hand side, by the
+    kernels that run it: pass_bytes for the z-first passes; for the x-first ones the x kernels
+    read or write the 3N vector and 3 Mx Ny Nz grid entries, the y kernels 3 Mx Nz (Ny + My),
+    the z kernel with the spectral product its grid of 3 Mx My Nz twice, the plane kernel
+    3 Mx Ny Nz twice, either with the canonical Green read of 6 Mx My Mz."""
+    if names[0] != "k_xfwd":
+        return pass_bytes(grid, Nx, Ny, Nz, N, s, names[1] == "-")
+    Mx, My, Mz = grid
+    x, green = 3 * N + 3 * Mx * Ny * Nz, 6 * Mx * My * Mz
+    if names[1] == "-":
+        return [x * s, 0, (6 * Mx * Ny * Nz + green) * s, x * s, 0]
+    y = 3 * Mx * Nz * (Ny + My)
+    return [x * s, y * s, (6 * Mx * My * Nz + green) * s, y * s, x * s]
+
+
 # GB300 FP64 (CUDA-core) rate, nominal: the measured-peaks file holds no FP64 figure
 FP64_NOMINAL_TFLOPS = 1.25
 
@@ -432,13 +448,17 @@ def time_batch(tdda, torch, w, incs, precision, steps, dev, flush_l2, keep_P=Fal
     return out, prof, n32
 
 
-def required_bytes(grid, Nx, N, s, fused, nrhs):
+def required_bytes(grid, Nx, N, s, fused, nrhs, names=None, Ny=0, Nz=0):
     """Bytes each kernel of one A-product over nrhs right-hand sides must move, as stored:
     the same grid and vector terms as pass_bytes, but the x pass reads the folded Green
     table (6 Hx Hy Hz entries, H = M/2 + 1) once per launch instead of the canonical
-    6 Mx My Mz.  Fused forms only (the compiled FP32 planes) and the five-pass form."""
+    6 Mx My Mz.  Fused forms only (the compiled FP32 planes) and the five-pass form; the
+    x-first kernels by their names."""
     Mx, My, Mz = grid
     H = (Mx // 2 + 1) * (My // 2 + 1) * (Mz // 2 + 1)
+    if names is not None and names[0] == "k_xfwd":
+        per = slot_bytes(names, grid, Nx, Ny, Nz, N, s)
+        return [(b - 6 * Mx * My * Mz * s) * nrhs + 6 * H * s if k == 2 else b * nrhs for k, b in enumerate(per)]
     plane = 3 * Nx * My * Mz
     if fused:
         zy = (3 * N + plane) * s * nrhs
@@ -447,11 +467,11 @@ def required_bytes(grid, Nx, N, s, fused, nrhs):
     return [per[0] * nrhs, per[1] * nrhs, (2 * plane * nrhs + 6 * H) * s, per[3] * nrhs, per[4] * nrhs]
 
 
-def pass_bytes_batch(w, grid, s, fused, nrhs):
+def pass_bytes_batch(w, grid, s, fused, nrhs, names=None):
     """Algorithmic bytes of each pass kernel of one A-product over nrhs right-hand sides:
     the grid and vector terms once per right-hand side, the Green read once per launch."""
     Mx, My, Mz = grid
-    per = pass_bytes(grid, w.Nx, w.Ny, w.Nz, w.N, s, fused)
+    per = slot_bytes(names or ["", "-" if fused else ""], grid, w.Nx, w.Ny, w.Nz, w.N, s)
     green = 6 * Mx * My * Mz * s
     return [(b - green) * nrhs + green if k == 2 else b * nrhs for k, b in enumerate(per)]
 
@@ -460,7 +480,7 @@ def pass_rooflines(w, grid, prof, names, s, fused, nrhs, peak):
     """Every pass kernel of one A-product against the HBM roof (the bytes each kernel must
     move, over its CUDA-event time), and the whole product on the canonical five-pass
     count (84 B + 48) N s, over the summed time of the kernels that run it."""
-    bk = pass_bytes_batch(w, grid, s, fused, nrhs)
+    bk = pass_bytes_batch(w, grid, s, fused, nrhs, names)
     passes = []
     live = [k for k, name in enumerate(names) if name not in ("", "-")]
     for k in live:
@@ -479,10 +499,10 @@ def batched_roofline(w, grid, prof, nrhs, s, peak, kernel, names):
     """Roofline of the x pass (the largest) for nrhs right-hand sides: the Green tensor is
     read once per launch, the grid once per right-hand side.  `passes` and `aproduct`
     give the other pass kernels and the whole product."""
-    b = pass_bytes_batch(w, grid, s, True, nrhs)[2]
+    b = pass_bytes_batch(w, grid, s, True, nrhs, names)[2]
     t = prof[2]
     ach = b / (t * 1e-3) / 1e9
-    req = required_bytes(grid, w.Nx, w.N, s, True, nrhs)[2]
+    req = required_bytes(grid, w.Nx, w.N, s, True, nrhs, names, w.Ny, w.Nz)[2]
     passes, whole = pass_rooflines(w, grid, prof, names, s, names[1] == "-", nrhs, peak)
     return {"kernel": kernel, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "algorithmic_bytes": b, "avg_ms": t, "required_bytes": req,
@@ -714,11 +734,11 @@ def run_ours(args, dist: Dist):
     pprec = tdda.FP32_REFINE if prec == "fp32" else tdda.FP64
     fused = core.pass_count(pprec) == 3
     names = pass_names(core, pprec)
-    bytes_k = pass_bytes(core.grid, w.Nx, w.Ny, w.Nz, w.N, s, fused)[k]
+    bytes_k = slot_bytes(names, core.grid, w.Nx, w.Ny, w.Nz, w.N, s)[k]
     t_k = (prof32 if prec == "fp32" else prof64)[k]
     peaks = measured_peaks()
     achieved = bytes_k / (t_k * 1e-3) / 1e9
-    req_k = required_bytes(core.grid, w.Nx, w.N, s, fused, 1)[k]
+    req_k = required_bytes(core.grid, w.Nx, w.N, s, fused, 1, names, w.Ny, w.Nz)[k]
     traffic = ncu_traffic(f"{names[k]}:{prec}:cfg2")
     names32 = pass_names(core, tdda.FP32_REFINE)
     passes32, whole32 = pass_rooflines(w, core.grid, prof32, names32, 8, core.pass_count(tdda.FP32_REFINE) == 3, 1,

@@ -334,25 +334,34 @@ tdda_status tdda_aproduct_noalloc(tdda_core* core, const double* b, double* y);
 tdda_status tdda_core_stream(const tdda_core* core, void** stream);
 /* Kernels this library has launched in this process (graph replays included). */
 unsigned long long tdda_kernel_launches(void);
-/* Average device time in ms of each of the five A-product passes (z forward,
- * y forward, x forward + spectral product + x inverse, y inverse, z inverse)
- * over `reps` plain products of nrhs right-hand sides, timed with CUDA events
+/* Average device time in ms of each of the five A-product passes (x forward, y
+ * forward, z forward + spectral product + z inverse, y inverse, x inverse; on
+ * grids without compiled axis kernels z forward, y forward, x forward + spectral
+ * product + x inverse, y inverse, z inverse) over `reps` plain products of nrhs right-hand sides, timed with CUDA events
  * on the core's stream. */
 tdda_status tdda_profile_aproduct(tdda_core* core, int precision, int nrhs, int reps, double* ms5);
 /* Kernels of one A-product at this precision: 5 (the passes above) or 3, when
- * the z and y passes are fused (FP32 on the compiled plane sizes).  With 3,
- * tdda_profile_aproduct reports the fused forward kernel in ms5[0], the fused
- * inverse in ms5[3], and ms5[1], ms5[4] hold only the gap between two events.
- * -1 for an invalid argument. */
+ * one kernel takes y, z and the spectral product of a plane, or the z and y
+ * passes are fused (FP32 on the compiled plane sizes).  With 3,
+ * tdda_profile_aproduct reports the first kernel in ms5[0], the middle one in
+ * ms5[2], the last in ms5[3], and ms5[1], ms5[4] hold only the gap between two
+ * events.  -1 for an invalid argument.  (tdda_aproduct itself sums FP64 products
+ * of up to 512 dipoles, 800 on grids without compiled axis kernels, directly in
+ * one kernel; TDDA_DIRECT=0 in the environment when the core is created keeps
+ * the passes.) */
 int tdda_core_pass_count(const tdda_core* core, int precision);
 /* Kernel that runs pass `pass` (0..4, the slots of tdda_profile_aproduct) at
- * this precision: "k_zfwd", "k_ypass", "k_xpass", "k_zinv", or with the
- * fused and register forms "k_zyfwd", "k_xpass2", "k_yzinv"; "" for a slot
- * that a fused kernel covers; NULL for an invalid argument.  Static string. */
+ * this precision: "k_xfwd", "k_yaxis", "k_zprod", "k_yaxis", "k_xinv", with
+ * whole planes in one block "k_xfwd", "", "k_xpass2", "k_xinv", ""; on grids
+ * without compiled axis kernels "k_zfwd", "k_ypass", "k_xpass", "k_zinv", or
+ * with the fused and register forms "k_zyfwd", "k_xpass2", "k_yzinv"; "" for a
+ * slot that a fused kernel covers; NULL for an invalid argument.  Static string. */
 const char* tdda_core_pass_name(const tdda_core* core, int precision, int pass);
 
-/* The FP32 x pass (x FFT, spectral product, inverse x FFT) of a core runs in
- * one of two forms: the register form on a two-stage radix plan (k_xpass2;
+/* Where the x-first product runs (all axes of compiled lengths), form 0 is that
+ * product with 8 or 16 lines a block of its gather (tile 0: built-in), form 1 the
+ * z-y-x passes with the shared-memory x pass.  Elsewhere the FP32 x pass (x FFT,
+ * spectral product, inverse x FFT) of a core runs in one of two forms: the register form on a two-stage radix plan (k_xpass2;
  * compiled for x lengths 32-192) with 8 or 16 z-columns a block, or the
  * shared-memory form on the length's compiled plan (k_xpass).  The tile does
  * not change results; the form changes the FFT's rounding (FP32 level).
