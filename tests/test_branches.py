@@ -63,3 +63,27 @@ def test_cross_lattice_models_of_one_core_equal_alone():
         m.close()
     for c in cores:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("box", [(40, 28, 12), (40, 32, 32), (40, 96, 10), (40, 64, 16), (40, 40, 24), (40, 48, 20)])
+def test_paired_plane_blocks_equal_alone(box):
+    """Batches of more than two planes an SM run the plane kernel with two blocks an SM (80 x 4
+    planes here), a right-hand side alone with one: bit by bit the same."""
+    if tdda.device_count() < 1:
+        pytest.skip("no CUDA device")
+    rng = np.random.Generator(np.random.PCG64(sum(box)))
+    R = lattice.bulk(*box)
+    core = tdda.AProductCore(*box, R, 10.0, 520.0, np.array([1.0, 2.25 + 0.05j]), max_rhs=4)
+    inc = list(lattice.config(3).incidences)[:4]
+    rho = np.repeat(0.4 + 0.2 * rng.random(R.size // 3), 3)
+    ms = [tdda.DDAModel(core, i.nK, i.E0, i.nE0, rho) for i in inc]
+    tdda.solve_batch(ms, tdda.FP32_REFINE, 60, 1e-6)
+    batch = [m.get_P() for m in ms]
+    for m, P in zip(ms, batch):
+        m.InitializeP()
+        tdda.solve_batch([m], tdda.FP32_REFINE, 60, 1e-6)
+        assert np.array_equal(m.get_P(), P)
+    for m in ms:
+        m.close()
+    core.close()

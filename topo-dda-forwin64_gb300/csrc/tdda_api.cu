@@ -584,12 +584,14 @@ template <typename T> int group_count(const tdda_core* c, int n) {
 // six pass events) is recorded for an ungrouped product only.
 template <typename T>
 cudaError_t aprod(tdda_core* c, int src, int snk, int n, const RhsVecs<T>* rhs, cudaEvent_t* ev = nullptr,
-                  int slot = 0, cudaStream_t stream = nullptr, long long grid_at = 0) {
+                  int slot = 0, cudaStream_t stream = nullptr, long long grid_at = 0, int batch = 0) {
     const int gs = group_size<T>(c, n);
+    Geom geom = c->g;
+    geom.batch = batch;
     for (int g0 = 0; g0 < n; g0 += gs) {
         count_launches(product_kernels<T>(c));
         const cudaError_t e = tdda::launch_aproduct<T>(
-            c->g, src, snk, std::min(gs, n - g0), rhs + g0, Prec<T>::green(c), Prec<T>::tw(c, 0), Prec<T>::tw(c, 1),
+            geom, src, snk, std::min(gs, n - g0), rhs + g0, Prec<T>::green(c), Prec<T>::tw(c, 0), Prec<T>::tw(c, 1),
             Prec<T>::tw(c, 2), c->cellmap, Prec<T>::grid(c) + grid_at, stream ? stream : c->stream,
             gs == n ? ev : nullptr, slot);
         if (e != cudaSuccess) return e;
@@ -612,16 +614,18 @@ template <typename T> int step_kernels(const tdda_core* c, int n) {
     return 2 * product_kernels<T>(c) * group_count<T>(c, n) * solve_branches<T>(c, n) + (kDeferred<T> ? 0 : 1);
 }
 
-// One step of the n right-hand sides from `first` on, on `stream`.
-template <typename T> cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStream_t stream) {
+// One step of the n right-hand sides from `first` on, on `stream`, of a batch of
+// `batch` whose other branches run beside it.
+template <typename T>
+cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStream_t stream, int batch) {
     const RhsVecs<T>* rhs = Prec<T>::rhs(c) + first;
     const long long at = first * grid_entries(c->g);
     cudaError_t e;
     if constexpr (kDeferred<T>) {
         // update, p, Ap
-        if ((e = aprod<T>(c, tdda::SRC_PUPD_DEF, tdda::SNK_AP, n, rhs, nullptr, slot, stream, at))) return e;
+        if ((e = aprod<T>(c, tdda::SRC_PUPD_DEF, tdda::SNK_AP, n, rhs, nullptr, slot, stream, at, batch))) return e;
         // alpha, t, At
-        return aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT_DEF, n, rhs, nullptr, slot, stream, at);
+        return aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT_DEF, n, rhs, nullptr, slot, stream, at, batch);
     } else {
         if ((e = aprod<T>(c, tdda::SRC_PUPD, tdda::SNK_AP, n, rhs))) return e;  // p, Ap, alpha
         if ((e = aprod<T>(c, tdda::SRC_TUPD, tdda::SNK_AT, n, rhs))) return e;  // t, At, zeta
@@ -694,7 +698,7 @@ cudaError_t enqueue_chunk(tdda_core* c, int n, const Branches& br, cudaGraphCond
         const int first = (int)((long long)n * b / br.count), end = (int)((long long)n * (b + 1) / br.count);
         if (e == cudaSuccess && b > 0) e = cudaStreamWaitEvent(br.s[b], br.fork, 0);
         for (int k = 0; k < kChunk && e == cudaSuccess; k++)
-            e = enqueue_iteration<T>(c, first, end - first, k & 1, br.s[b]);
+            e = enqueue_iteration<T>(c, first, end - first, k & 1, br.s[b], br.count > 1 ? n : 0);
         if (e == cudaSuccess && b > 0) e = cudaEventRecord(br.join[b], br.s[b]);
     }
     for (int b = 1; b < br.count && e == cudaSuccess; b++) e = cudaStreamWaitEvent(c->stream, br.join[b], 0);

@@ -924,6 +924,9 @@ template <int MY, int MZ> struct Plane {
     // Registers are given to warps in fours, one per SM quarter: 512 threads may
     // use 128, which phase 3 needs.
     static constexpr int NT = MY * MZ <= 1024 ? 256 : 512;
+    // a second form with two blocks of 256 threads an SM, where both fit: it overlaps
+    // the phases of two planes, but takes longer over one (PlaneLaunch)
+    static constexpr bool kPair = NT == 512 && smem <= 113000;
 };
 constexpr size_t kMaxPlaneSmem = 232448;  // 227 KB, the most one block may use
 template <int MY, int MZ> constexpr bool plane_fits() { return Plane<MY, MZ>::smem <= kMaxPlaneSmem; }
@@ -965,8 +968,8 @@ __device__ __forceinline__ void prefetch_plane(const Geom& g, const RhsVecs<floa
     if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a16), "r"(bytes) : "memory");
 }
 
-template <int MY, int MZ>
-__global__ void __launch_bounds__(Plane<MY, MZ>::NT) k_xpass2p(Geom g, const RhsVecs<float>* __restrict__ rhs,
+template <int MY, int MZ, int NT>
+__global__ void __launch_bounds__(NT, NT < Plane<MY, MZ>::NT ? 2 : 0) k_xpass2p(Geom g, const RhsVecs<float>* __restrict__ rhs,
                                                                 const float2* __restrict__ green,
                                                                 const float2* __restrict__ twy,
                                                                 const float2* __restrict__ twz,
@@ -975,7 +978,7 @@ __global__ void __launch_bounds__(Plane<MY, MZ>::NT) k_xpass2p(Geom g, const Rhs
     using PL = Plane<MY, MZ>;
     using Y = typename PL::Y;
     using Z = typename PL::Z;
-    constexpr int NT = PL::NT, ZP = PL::ZP, LZ = Z::LX;
+    constexpr int ZP = PL::ZP, LZ = Z::LX;
     constexpr int B1 = Y::R1, B2 = Y::R2, BH = Y::RH, A1 = Z::R1, A2 = Z::R2, AH = Z::RH;
     constexpr int CS = MY * ZP;  // from component to component
     static_assert(B2 == 8 && A2 % 2 == 0, "plans of the plane");
@@ -1228,11 +1231,30 @@ template <typename T, int M> struct ZprodLaunch {
 
 template <int MY, int MZ> struct PlaneLaunch {
     using PL = Plane<MY, MZ>;
-    static cudaError_t run(const PassArgs<float>& a) {
-        return launch_axis(a, k_xpass2p<MY, MZ>, dim3(a.g.px.M, a.nrhs), PL::NT, PL::smem, a.rhs, a.green, a.twy, a.twz,
-                           a.grid);
+    template <int NT> static cudaError_t run1(const PassArgs<float>& a) {
+        return launch_axis(a, k_xpass2p<MY, MZ, NT>, dim3(a.g.px.M, a.nrhs), NT, PL::smem, a.rhs, a.green, a.twy,
+                           a.twz, a.grid);
     }
-    static cudaError_t configure() { return allow_smem((const void*)k_xpass2p<MY, MZ>, PL::smem); }
+    // Pairs of blocks where the planes that run side by side (the batch's, over its
+    // branches) are more than two an SM: steps of 40 x 40 x 12, eight right-hand sides
+    // 75 -> 64 us, of 45 x 33 x 19, four 65 -> 59, of 64 x 64 x 16, four 83 -> 76 and
+    // eight 157 -> 144; below, a plane's own time counts (64 x 64 x 16, one 34 -> 40,
+    // two 49 -> 54 with pairs).
+    static cudaError_t run(const PassArgs<float>& a) {
+        if constexpr (PL::kPair) {
+            const int sms = a.g.sms > 0 ? a.g.sms : 152;
+            const long long planes = (long long)a.g.px.M * std::max(a.nrhs, a.g.batch);
+            if (planes > 2LL * sms) return run1<256>(a);
+        }
+        return run1<PL::NT>(a);
+    }
+    static cudaError_t configure() {
+        cudaError_t e = allow_smem((const void*)k_xpass2p<MY, MZ, PL::NT>, PL::smem);
+        if constexpr (PL::kPair) {
+            if (e == cudaSuccess) e = allow_smem((const void*)k_xpass2p<MY, MZ, 256>, PL::smem);
+        }
+        return e;
+    }
 };
 
 }  // namespace dev

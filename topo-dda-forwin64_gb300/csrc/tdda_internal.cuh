@@ -55,6 +55,7 @@ struct Geom {
                        // 1 the next kernel released after the wait; 2 before the last
                        // stage; 3 per launch: 1 for at most `sms` blocks, else 2
     int sms;           // streaming multiprocessors of the core's device
+    int batch = 0;     // right-hand sides that run beside a launch's own, its own included (0: none)
 };
 
 // The release point of an early launch of `blocks` blocks.  Released right after
