@@ -644,8 +644,8 @@ cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStre
 //  - one where all planes fit one wave (13 x 100 x 9, four: 37.5 us, in two 38.1);
 //  - four (of one right-hand side or more) where two right-hand sides are about a
 //    wave, which halves would overshoot, up to five waves (37 x 51 x 13, four:
-//    71 us, in two 74, in four 65; 40 x 40 x 12, eight: 78, 79 and 76, but
-//    twelve, 6.3 waves: 106, 101 and 108);
+//    71 us, in two 74, in four 66; 40 x 40 x 12, eight: 70, 68 and 64, but
+//    twelve, 6.3 waves: 94, 84 and 91);
 //  - three for three (80 x 80 x 20: 141 us, in two 134, in three 131);
 //  - one for plane blocks that take nearly all of an SM's shared memory where the
 //    last wave is nearly full or the launch long, whose tails are short beside what
