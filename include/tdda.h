@@ -358,21 +358,23 @@ int tdda_core_pass_count(const tdda_core* core, int precision);
  * slot that a fused kernel covers; NULL for an invalid argument.  Static string. */
 const char* tdda_core_pass_name(const tdda_core* core, int precision, int pass);
 
-/* Where the x-first product runs (all axes of compiled lengths), form 0 is that
- * product with 8 or 16 lines a block of its gather (tile 0: built-in), form 1 the
- * z-y-x passes with the shared-memory x pass.  Elsewhere the FP32 x pass (x FFT,
- * spectral product, inverse x FFT) of a core runs in one of two forms: the register form on a two-stage radix plan (k_xpass2;
- * compiled for x lengths 32-192) with 8 or 16 z-columns a block, or the
- * shared-memory form on the length's compiled plan (k_xpass).  The tile does
- * not change results; the form changes the FFT's rounding (FP32 level).
- * form 0: register form where compiled, tile 8, 16 or 0 (built-in: 16 for
- * x length 128, else 8); form 1: shared-memory form, tile 0.  Captured FP32
+/* Two forms of the FP32 product of a core, at FFT x lengths with a register form
+ * of the x pass (x FFT, spectral product, inverse x FFT; compiled for 32-192).
+ * Where the x-first product runs (all axes of compiled lengths), form 0 is that
+ * product, with 8 or 16 lines a block of its gather, and form 1 the z-y-x passes
+ * with the shared-memory x pass (k_xpass).  Elsewhere form 0 is the register form
+ * of the x pass (k_xpass2) with 8 or 16 z-columns a block, form 1 the
+ * shared-memory form on the length's compiled plan.  At x lengths without a
+ * register form both forms are the same product: the x-first one where it runs,
+ * else the passes with the shared-memory x pass.  The tile does not change
+ * results; the form changes the FFT's rounding (FP32 level).
+ * form 0: tile 8, 16 or 0 (built-in); form 1: tile 0.  Captured FP32
  * solve steps of the core are dropped and captured again on next use; the
  * call waits for the core's stream first. */
 tdda_status tdda_core_set_xpass(tdda_core* core, int form, int tile);
 typedef struct {
     int x_form, x_tile;  /* the chosen configuration (now set on the core) */
-    int ncand;           /* candidates timed: 3, or 1 where the x length has no register form */
+    int ncand;           /* candidates timed: 3, or 1 (form 1) where the x length has no register form */
     int form[4], tile[4];
     double ms[4];        /* average ms of one FP32 A-product of nrhs right-hand sides, per candidate */
 } tdda_xpass_tune;

@@ -2609,8 +2609,8 @@ tdda_status tdda_core_autotune(tdda_core* c, int nrhs, int reps, tdda_xpass_tune
     }
     TDDA_TRY(set_device(c->device));
     *out = tdda_xpass_tune{};
-    // candidates: the register form with 8 and 16 z-columns a block, where the
-    // x length has a two-stage plan, and the shared-memory form
+    // candidates: form 0 with 8 and 16 lines or z-columns a block, where the x
+    // length has two forms, and form 1
     int nc = 0;
     if (tdda::xpass2_length(c->g.px.M)) {
         out->form[nc] = 0, out->tile[nc++] = 8;

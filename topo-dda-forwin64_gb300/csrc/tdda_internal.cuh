@@ -45,7 +45,8 @@ struct Geom {
     // FP32 x pass (set by tdda_core_set_xpass / tdda_core_autotune):
     int x_form;        // 0: the x-first product where its lengths are compiled, else the
                        // register form on a two-stage plan where one is compiled;
-                       // 1: the shared-memory form on the length's compiled plan
+                       // 1: the shared-memory form on the length's compiled plan, where
+                       // the length has a register form (elsewhere as 0)
     int x_tile;        // lines per block of the x-first gather, or z-columns per block of
                        // the register form: 8, 16, or 0 for the built-in choice
     int multi;         // 1: a cross-lattice batch -- every right-hand side brings its own

@@ -903,9 +903,14 @@ cudaError_t launch_aproduct_ext(const Geom& g, const RhsVecs<T>* rhs, const doub
 
 // The x-first product where its lengths are compiled (FP32: in its plane form
 // where the plane fits a block, unless the shared-memory x pass is asked for),
-// else the z-y-x passes, fused where compiled.
+// else the z-y-x passes, fused where compiled.  The two forms of Geom::x_form
+// differ where the x pass has a register form to be the other of; at the other
+// x lengths (12 to 25, 224, 256) they are one, and the x-first product is the
+// faster one everywhere (z-y-x and x-first, us a product: 128 x 128 x 32 338 and
+// 125, 112 x 40 x 20 98 and 34, 12 x 40 x 20 68 and 24, 13 x 13 x 13 65 and 23).
 ProductForm product_form(const Geom& g, bool fp32) {
-    if (axes_lengths(g) && !g.passes && (!fp32 || g.x_form == 0)) return fp32 && axes_plane(g) ? FORM_PLANE : FORM_AXES;
+    const bool passes = g.passes || (fp32 && g.x_form == 1 && xpass2_length(g.px.M));
+    if (axes_lengths(g) && !passes) return fp32 && axes_plane(g) ? FORM_PLANE : FORM_AXES;
     return zy_fused(g, fp32) ? FORM_FUSED_ZY : FORM_PASSES;
 }
 

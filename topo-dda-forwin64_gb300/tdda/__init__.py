@@ -303,8 +303,9 @@ class AProductCore:
         return out
 
     def set_xpass(self, form: int, tile: int = 0):
-        """FP32 x-pass configuration: form 0 = register form (tile 8, 16, or 0 for the
-        built-in choice), form 1 = shared-memory form (tile 0)."""
+        """FP32 product: form 0 = the x-first product or the register form of the x pass (tile 8, 16,
+        or 0 for the built-in choice), form 1 = the shared-memory form (tile 0); one and the same at
+        x lengths without a register form."""
         _check(load().tdda_core_set_xpass(self.h, int(form), int(tile)), "tdda_core_set_xpass")
 
     def autotune(self, nrhs: int = 1, reps: int = 10) -> dict:
