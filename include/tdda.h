@@ -396,11 +396,15 @@ typedef struct {
     int group;           /* the chosen right-hand sides per launch (0: all; now set on the core) */
     int ncand;           /* candidates timed: 0, nrhs / 2, nrhs / 4, ... (at most 4) */
     int groups[4];
-    double ms[4];        /* average ms of one FP32 A-product of nrhs right-hand sides, per candidate */
+    double ms[4];        /* average ms of half an FP32 step of nrhs right-hand sides (one product with its
+                          * vector updates), per candidate */
 } tdda_batch_tune;
-/* Autotuner of the batch schedule: times `reps` plain FP32 A-products of nrhs
- * right-hand sides (CUDA events, after one warm-up) for each candidate group
- * size and sets the fastest on the core. */
+/* Autotuner of the batch schedule: times FP32 solver steps of nrhs right-hand
+ * sides (at least `reps` products; CUDA events, after a warm-up) for each
+ * candidate group size, as a solve runs them (the whole batch in its parallel
+ * branches), and sets the fastest on the core.  The steps run on models of a
+ * plane wave that the call makes and frees (their device memory is that of nrhs
+ * models of a refined solve). */
 tdda_status tdda_core_autotune_batch(tdda_core* core, int nrhs, int reps, tdda_batch_tune* out);
 
 #ifdef __cplusplus

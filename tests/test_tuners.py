@@ -30,3 +30,51 @@ def test_x_lengths_of_one_form_keep_their_product(box):
         assert c.pass_names(tdda.FP32_REFINE) == names
         assert np.array_equal(c.Aproduct(b, precision=tdda.FP32_REFINE), y)
     c.close()
+
+
+# box, right-hand sides: the number of branches of a solve's steps there on 152 SMs
+BRANCHES = [((20, 20, 10), 3, 1), ((48, 6, 6), 2, 2), ((48, 6, 6), 7, 2), ((48, 6, 6), 3, 3), ((20, 20, 10), 5, 4),
+            ((20, 20, 10), 8, 4)]
+
+
+def _core(box, n):
+    if tdda.device_count() < 1:
+        pytest.skip("no CUDA device")
+    R = lattice.bulk(*box)
+    return tdda.AProductCore(*box, R, 10.0, 520.0, MAT, max_rhs=n), R
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("loop", ["1", "0"])
+@pytest.mark.parametrize("box,n,branches", BRANCHES)
+def test_batch_tuner_times_the_branches_of_a_solve(box, n, branches, loop, monkeypatch):
+    """The candidates are timed on solver steps, the whole batch in its branches: by the kernels that
+    eight more steps of each launch (twelve steps against four where 24 and 8 products are asked for)."""
+    monkeypatch.setenv("TDDA_DEVICE_LOOP", loop)
+    core, _ = _core(box, n)
+
+    def tune(reps):
+        before = tdda.kernel_launches()
+        t = core.autotune_batch(nrhs=n, reps=reps)
+        assert t["group"] == min(t["candidates"], key=lambda k: k["ms"])["group"]
+        assert all(k["ms"] > 0 for k in t["candidates"])
+        return tdda.kernel_launches() - before, [k["group"] for k in t["candidates"]]
+
+    tune(8)
+    (few, groups), (many, _) = tune(8), tune(24)
+    sets = [branches if g == 0 else -(-n // g) for g in groups]
+    ends = 2  # the step end after every fourth step
+    assert groups[0] == 0
+    assert many - few == 16 * core.pass_count(tdda.FP32_REFINE) * sum(sets) + ends * len(groups)
+    core.close()
+
+
+@pytest.mark.gpu
+def test_batch_tuner_of_a_core_of_one_material():
+    """Such a core has no models; its products are timed."""
+    if tdda.device_count() < 1:
+        pytest.skip("no CUDA device")
+    c = tdda.AProductCore(9, 8, 7, lattice.bulk(9, 8, 7), 10.0, 520.0, MAT[:1], max_rhs=2)
+    t = c.autotune_batch(nrhs=2, reps=2)
+    assert [k["group"] for k in t["candidates"]] == [0, 1] and all(k["ms"] > 0 for k in t["candidates"])
+    c.close()

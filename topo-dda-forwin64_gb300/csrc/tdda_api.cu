@@ -2560,6 +2560,64 @@ tdda_status profile_products(tdda_core* c, int precision, int nrhs, int reps, do
     return st;
 }
 
+// Models for timing a batch's steps on a core: a plane wave on a structure half way
+// between the first two materials.
+struct TimedBatch {
+    std::vector<tdda_model*> ms;
+    tdda_status create(tdda_core* c, int n) {
+        const double nK[3] = {0, 0, 1}, nE0[3] = {1, 0, 0};
+        const std::vector<double> rho(3 * (size_t)c->N, 0.5);
+        std::vector<RhsVecs<float>> h32(n);
+        for (int i = 0; i < n; i++) {
+            tdda_model* m = nullptr;
+            TDDA_TRY(tdda_model_create(c, nK, 1.0, nE0, rho.data(), &m));
+            ms.push_back(m);
+            TDDA_TRY(model_alloc_f32(m));
+            TDDA_CK1(tdda::launch_to_f32(3 * c->N, m->E, m->fE, c->stream));
+            TDDA_CK1(tdda::launch_zero<float>(3LL * c->N, m->fP, c->stream));
+            h32[i] = vecs32(c, m, i);
+        }
+        TDDA_CK(cudaMemcpyAsync(c->rhs32, h32.data(), sizeof(RhsVecs<float>) * n, cudaMemcpyHostToDevice, c->stream));
+        return TDDA_OK;
+    }
+    ~TimedBatch() {
+        for (tdda_model* m : ms) tdda_model_destroy(m);
+    }
+};
+
+// Half the device time in ms of one FP32 solver step of the models (its two
+// products with their vector updates), in the core's batch schedule: at least
+// `reps` products, as the difference of two runs, so that neither what a solve
+// does before and after its steps nor the graph's capture counts.  (Plain products
+// leave out the vectors, beside which no group's work grid stays in L2: 96 x 96 x 24,
+// eight right-hand sides, in one launch or by twos 249 and 248 us a product, but 602
+// and 687 us a step.)
+tdda_status time_steps(tdda_core* c, std::vector<tdda_model*>& ms, int reps, double* out) {
+    const int n = (int)ms.size();
+    const int runs[3] = {kChunk, kChunk, kChunk + kChunk * ((reps - 1) / (2 * kChunk) + 1)};  // steps: warm-up, two timed
+    cudaEvent_t ev[2] = {};
+    for (cudaEvent_t& e : ev) TDDA_CK(cudaEventCreate(&e));
+    float t[3] = {};
+    int it[3] = {};
+    tdda_status st = TDDA_OK;
+    for (int k = 0; k < 3 && st == TDDA_OK; k++) {
+        for (int i = 0; i < n; i++) c->hst[i] = fresh_state(0.0, runs[k], 0);
+        cudaError_t e = cudaMemcpyAsync(c->st32, c->hst, sizeof(SolveState) * n, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[0], c->stream);
+        if (e == cudaSuccess) st = krylov<float>(c, n, true, runs[k]);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[1], c->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&t[k], ev[0], ev[1]);
+        if (e != cudaSuccess && st == TDDA_OK) st = cuda_fail(e, "timed steps");
+        it[k] = c->hst[0].it;
+    }
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+    // a solve that ends by itself (converged to the last bit, or not finite) takes the same
+    // steps in every schedule
+    *out = it[2] > it[1] ? (t[2] - t[1]) / (2.0 * (it[2] - it[1])) : t[2] / (2.0 * std::max(1, it[2]));
+    return st;
+}
+
 // A captured solve step holds its pass kernels and their Geom: a new FP32 x-pass
 // configuration drops the FP32 step graphs (captured again on next use).
 tdda_status set_xpass(tdda_core* c, int form, int tile) {
@@ -2659,16 +2717,22 @@ tdda_status tdda_core_autotune_batch(tdda_core* c, int nrhs, int reps, tdda_batc
         if (g < nrhs) out->groups[nc++] = g;
     out->ncand = nc;
     const int group0 = c->group;
+    const bool models = c->nmat > 1;  // a core of one material takes products only
+    TimedBatch b;
+    if (models) TDDA_TRY(b.create(c, nrhs));
     int best = -1;
     for (int k = 0; k < nc; k++) {
-        double ms5[5];
         tdda_status st = set_batch_group(c, out->groups[k]);
-        if (st == TDDA_OK) st = profile_products(c, TDDA_FP32_REFINE, nrhs, reps, ms5);
+        if (st == TDDA_OK && models) st = time_steps(c, b.ms, reps, &out->ms[k]);
+        if (st == TDDA_OK && !models) {
+            double ms5[5];
+            st = profile_products(c, TDDA_FP32_REFINE, nrhs, reps, ms5);
+            if (st == TDDA_OK) out->ms[k] = ms5[0] + ms5[1] + ms5[2] + ms5[3] + ms5[4];
+        }
         if (st != TDDA_OK) {
             set_batch_group(c, group0);
             return st;
         }
-        out->ms[k] = ms5[0] + ms5[1] + ms5[2] + ms5[3] + ms5[4];
         if (best < 0 || out->ms[k] < out->ms[best]) best = k;
     }
     out->group = out->groups[best];

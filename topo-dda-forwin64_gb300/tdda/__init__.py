@@ -320,7 +320,8 @@ class AProductCore:
         _check(load().tdda_core_set_batch_group(self.h, int(group)), "tdda_core_set_batch_group")
 
     def autotune_batch(self, nrhs: int, reps: int = 5) -> dict:
-        """Time the batch-schedule candidates on this core's FP32 A-product and keep the fastest."""
+        """Time the batch-schedule candidates on FP32 solver steps of this core and keep the fastest
+        (ms: half a step, one product with its vector updates)."""
         t = BatchTune()
         _check(load().tdda_core_autotune_batch(self.h, int(nrhs), int(reps), ctypes.byref(t)),
                "tdda_core_autotune_batch")
