@@ -78,3 +78,34 @@ def test_batch_tuner_of_a_core_of_one_material():
     t = c.autotune_batch(nrhs=2, reps=2)
     assert [k["group"] for k in t["candidates"]] == [0, 1] and all(k["ms"] > 0 for k in t["candidates"])
     c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("box,n,branches", BRANCHES)
+def test_solves_run_in_their_branches(box, n, branches, monkeypatch):
+    """The number of branches of a solve's steps: the kernels that eight more steps launch, beside
+    those of eight more steps with a launch for each right-hand side."""
+    monkeypatch.setenv("TDDA_DEVICE_LOOP", "0")
+    core, R = _core(box, n)
+    rng = np.random.Generator(np.random.PCG64(n))
+    inc = (list(lattice.config(3).incidences) * 2)[:n]
+    ms = [tdda.DDAModel(core, i.nK, i.E0, i.nE0, np.repeat(rng.random(R.size // 3), 3)) for i in inc]
+    tdda.solve_batch(ms, tdda.FP32_REFINE, 4, 1e-30)  # what a core and its models make once
+
+    def launched(steps):
+        for m in ms:
+            m.InitializeP()
+        before = tdda.kernel_launches()
+        tdda.solve_batch(ms, tdda.FP32_REFINE, steps, 1e-30)
+        return tdda.kernel_launches() - before
+
+    more = {}
+    for group in (0, 1):
+        core.set_batch_group(group)
+        more[group] = launched(12) - launched(4)
+    ends = 2  # the step end after every fourth step
+    assert more[1] == 16 * core.pass_count(tdda.FP32_REFINE) * n + ends
+    assert more[0] == 16 * core.pass_count(tdda.FP32_REFINE) * branches + ends
+    for m in ms:
+        m.close()
+    core.close()
