@@ -1333,16 +1333,21 @@ tdda_status upload_subset(Shape* s, const std::vector<int>& ks) {
 }  // namespace
 
 double core_bytes(int Nx, int Ny, int Nz, int N, int max_rhs) {
-    const double Mx = fft_length(Nx, false), My = fft_length(Ny, false), Mz = fft_length(Nz, true);
-    const double H = (Mx / 2 + 1) * (My / 2 + 1) * (Mz / 2 + 1);
-    const double n3 = 3.0 * N;
-    // FFT work grid entries: x kept to the lattice, or z (the x-first product)
-    const double grid = 3.0 * My * std::max((double)Nx * Mz, Mx * Nz) * max_rhs;
+    Geom g{};
+    g.Nx = Nx, g.Ny = Ny, g.Nz = Nz, g.N = N;
+    if (!make_plan(fft_length(Nx, false), &g.px) || !make_plan(fft_length(Ny, false), &g.py) ||
+        !make_plan(fft_length(Nz, true), &g.pz))
+        return 0.0;  // core_create refuses it
+    grid_layout(&g);
+    const double H = (double)g.Hx * g.Hy * g.Hz, n3 = 3.0 * N;
+    const double grid = (double)grid_entries(g) * max_rhs;                  // FFT work grids
+    const double octant = 6.0 * Nx * ((double)Ny * g.Hz + (double)g.Hy * g.Hz);  // scratch while the core is built
+    const double table = direct_products(g) ? 6.0 * Nx * Ny * Nz : 0.0;     // direct products
     return (double)Nx * Ny * Nz * 4 + n3 * 4           // cellmap, R
            + 6 * H * (16 + 8 + 16)                     // Green spectra (FP64, FP32, double-float)
            + grid * (16 + 8)                           // FP64 and FP32 grids
            + n3 * 2 * (16 + 8)                         // product staging
-           + 6 * Mx * My * Mz * 16                     // scratch while the core is built (at most), direct table
+           + (octant + table) * 16
            + 1e6;                                      // reduction partials, states, twiddles
 }
 
