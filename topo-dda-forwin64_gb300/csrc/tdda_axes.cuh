@@ -953,12 +953,12 @@ template <int MY> __device__ __forceinline__ int mirrored_row(int i) {
     return i % 16 < 8 ? h : (h == 0 ? MY / 2 : MY - h);
 }
 
-// The plane of the block that follows this one on its SM (one block fills an
-// SM, and blocks start in order) into L2: with a batch the work grid does not
-// stay there, and phase 1 would wait for DRAM at the start of every block.
+// The plane of the block that follows this one on its SM (`resident` blocks fill
+// the device, and blocks start in order) into L2: with a batch the work grid does
+// not stay there, and phase 1 would wait for DRAM at the start of every block.
 __device__ __forceinline__ void prefetch_plane(const Geom& g, const RhsVecs<float>* rhs, const float2* grid, int kx,
-                                               int b) {
-    kx += g.sms;
+                                               int b, int resident) {
+    kx += resident;
     while (kx >= g.px.M) kx -= g.px.M, b++;
     if (b >= (int)gridDim.y) return;
     const long long n = 3LL * (g.multi ? rhs[b].Ny : g.Ny) * (g.multi ? rhs[b].Nz : g.Nz);
@@ -996,7 +996,13 @@ __global__ void __launch_bounds__(NT, NT < Plane<MY, MZ>::NT ? 2 : 0) k_xpass2p(
     float2* gp = grid + (long long)b * g.vb + (long long)kx * 3 * Ny * Nz;
     grid_dep_wait();
     if (g.early == 1) grid_dep_release();
-    if (threadIdx.x == 0) prefetch_plane(g, rhs, grid, kx, b);
+    // not for the small planes, which are several to an SM and whose grid stays in L2 (a
+    // prefetch of planes that already run: 64 x 16 x 16, sixteen right-hand sides 107.5 us a
+    // step with it, 105.2 without; 40 x 20 x 10 61.9 and 60.7); in pairs the next plane is two
+    // blocks an SM away (13 batches: within 0.6% of the distance of one, either way)
+    if constexpr (PL::NT == 512) {
+        if (threadIdx.x == 0) prefetch_plane(g, rhs, grid, kx, b, NT < PL::NT ? 2 * g.sms : g.sms);
+    }
     // 1: rows y = jj + 8 r < Ny of column z
     for (int w = threadIdx.x; w < 3 * B2 * LZ; w += NT) {
         const int z = w % LZ, jj = (w / LZ) % B2, c = w / (LZ * B2);
