@@ -242,7 +242,7 @@ __device__ __forceinline__ int fold(int k, int M) { return 2 * k > M ? M - k : k
 
 // The six components at folded point (fy, fx, fz).  The FP32 table holds them as
 // three planes of component pairs (xx|xy, xz|yy, yz|zz), read as 16-byte values;
-// the FP64 and double-float tables hold 16-byte components.  The strides put the
+// the FP64 table holds 16-byte components.  The strides put the
 // axis that the threads of a warp walk innermost (GreenStride), so that a warp's
 // loads read whole lines.
 template <typename T>
@@ -256,10 +256,6 @@ __device__ __forceinline__ void load_green(const cx<T>* green, const Geom& g, in
         a0 = mk<T>(u.x, u.y); a1 = mk<T>(u.z, u.w);
         a2 = mk<T>(v.x, v.y); a3 = mk<T>(v.z, v.w);
         a4 = mk<T>(w.x, w.y); a5 = mk<T>(w.z, w.w);
-    } else if constexpr (is_dd<T>) {
-        const float4* q = reinterpret_cast<const float4*>(green) + at;
-        a0 = dd2(__ldg(q)); a1 = dd2(__ldg(q + gs.l)); a2 = dd2(__ldg(q + 2 * gs.l));
-        a3 = dd2(__ldg(q + 3 * gs.l)); a4 = dd2(__ldg(q + 4 * gs.l)); a5 = dd2(__ldg(q + 5 * gs.l));
     } else {
         const cx<T>* q = green + at;
         a0 = __ldg(q); a1 = __ldg(q + gs.l); a2 = __ldg(q + 2 * gs.l);
