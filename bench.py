@@ -213,7 +213,10 @@ def ncu_traffic(key):
 
 def pass_names(core, precision):
     """Kernel of each profile slot, from the library ("-" where a fused kernel covers it)."""
-    return [n or "-" for n in core.pass_names(precision)]
+    names = [n or "-" for n in core.pass_names(precision)]
+    if names[0] == "k_xfwd" and names[2] == "k_xpass2":  # the library's name of the x-first plane kernel
+        names[2] = "k_xpass2p"
+    return names
 
 
 # ------------------------------------------------------------------ CPU baseline

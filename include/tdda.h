@@ -337,8 +337,8 @@ unsigned long long tdda_kernel_launches(void);
 /* Average device time in ms of each of the five A-product passes (x forward, y
  * forward, z forward + spectral product + z inverse, y inverse, x inverse; on
  * grids without compiled axis kernels z forward, y forward, x forward + spectral
- * product + x inverse, y inverse, z inverse) over `reps` plain products of nrhs right-hand sides, timed with CUDA events
- * on the core's stream. */
+ * product + x inverse, y inverse, z inverse) over `reps` plain products of nrhs
+ * right-hand sides, timed with CUDA events on the core's stream. */
 tdda_status tdda_profile_aproduct(tdda_core* core, int precision, int nrhs, int reps, double* ms5);
 /* Kernels of one A-product at this precision: 5 (the passes above) or 3, when
  * one kernel takes y, z and the spectral product of a plane, or the z and y
@@ -352,7 +352,8 @@ tdda_status tdda_profile_aproduct(tdda_core* core, int precision, int nrhs, int 
 int tdda_core_pass_count(const tdda_core* core, int precision);
 /* Kernel that runs pass `pass` (0..4, the slots of tdda_profile_aproduct) at
  * this precision: "k_xfwd", "k_yaxis", "k_zprod", "k_yaxis", "k_xinv", with
- * whole planes in one block "k_xfwd", "", "k_xpass2", "k_xinv", ""; on grids
+ * whole planes in one block "k_xfwd", "", "k_xpass2", "k_xinv", "" (the plane
+ * kernel, k_xpass2p in a profiler; after "k_xfwd" the name stands for it); on grids
  * without compiled axis kernels "k_zfwd", "k_ypass", "k_xpass", "k_zinv", or
  * with the fused and register forms "k_zyfwd", "k_xpass2", "k_yzinv"; "" for a
  * slot that a fused kernel covers; NULL for an invalid argument.  Static string. */

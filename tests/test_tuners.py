@@ -33,8 +33,8 @@ def test_x_lengths_of_one_form_keep_their_product(box):
 
 
 # box, right-hand sides: the number of branches of a solve's steps there on 152 SMs
-BRANCHES = [((20, 20, 10), 3, 1), ((48, 6, 6), 2, 2), ((48, 6, 6), 7, 2), ((48, 6, 6), 3, 3), ((20, 20, 10), 5, 4),
-            ((20, 20, 10), 8, 4)]
+BRANCHES = [((20, 20, 10), 3, 1), ((48, 6, 6), 2, 2), ((48, 6, 6), 7, 2), ((48, 6, 6), 3, 3), ((20, 20, 10), 5, 2),
+            ((20, 20, 10), 8, 2), ((20, 24, 20), 5, 4), ((33, 24, 12), 4, 4)]
 
 
 def _core(box, n):
@@ -106,6 +106,28 @@ def test_solves_run_in_their_branches(box, n, branches, monkeypatch):
     ends = 2  # the step end after every fourth step
     assert more[1] == 16 * core.pass_count(tdda.FP32_REFINE) * n + ends
     assert more[0] == 16 * core.pass_count(tdda.FP32_REFINE) * branches + ends
+    for m in ms:
+        m.close()
+    core.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("loop", ["1", "0"])
+@pytest.mark.parametrize("box,n", [((20, 24, 20), 5), ((33, 24, 12), 4), ((25, 26, 11), 6)])
+def test_four_branches_equal_alone(box, n, loop, monkeypatch):
+    """Four branches, of equal and unequal shares: each solution bit by bit the one solved alone."""
+    monkeypatch.setenv("TDDA_DEVICE_LOOP", loop)
+    core, R = _core(box, n)
+    rng = np.random.Generator(np.random.PCG64(sum(box)))
+    inc = (list(lattice.config(3).incidences) * 2)[:n]
+    ms = [tdda.DDAModel(core, i.nK, i.E0, i.nE0, np.repeat(rng.random(R.size // 3), 3)) for i in inc]
+    infos = tdda.solve_batch(ms, tdda.FP32_REFINE, 400, 1e-8)
+    batch = [m.get_P() for m in ms]
+    for k, m in enumerate(ms):
+        m.InitializeP()
+        [alone] = tdda.solve_batch([m], tdda.FP32_REFINE, 400, 1e-8)
+        assert alone["inner_iterations"] == infos[k]["inner_iterations"]
+        assert np.array_equal(m.get_P(), batch[k])
     for m in ms:
         m.close()
     core.close()

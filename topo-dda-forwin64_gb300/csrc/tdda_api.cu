@@ -646,6 +646,11 @@ cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStre
 //    wave, which halves would overshoot, up to five waves (37 x 51 x 13, four:
 //    71 us, in two 74, in four 66; 40 x 40 x 12, eight: 70, 68 and 64, but
 //    twelve, 6.3 waves: 94, 84 and 91);
+//    Not for planes of up to 1024 points, which run several to an SM: steps in two
+//    branches take 0.95 to 1.06 times those in four there, 1.00 in the mean (18
+//    lattices and counts; 20 x 20 x 10, four: 26.0 and 25.9 us), and the graph of
+//    four costs a new core 0.2 to 0.3 ms more (a core, its models and a solve of six
+//    preconditioned steps, 18 x 16 x 8, four: 1638 us in four, 1328 in two);
 //  - three for three (80 x 80 x 20: 141 us, in two 134, in three 131);
 //  - one for plane blocks that take nearly all of an SM's shared memory where the
 //    last wave is nearly full or the launch long, whose tails are short beside what
@@ -661,7 +666,8 @@ template <typename T> int solve_branches(const tdda_core* c, int n) {
     if (planes <= sms) return 1;
     if (form == tdda::FORM_PLANE && plane_bytes > 200 * 1024 && (planes > 7 * sms || 20 * (planes % sms) > 17 * sms))
         return 1;
-    if (20LL * g.px.M <= 11 * sms && planes <= 5 * sms) return std::min(n, kMaxBranches);
+    const bool small = g.py.M * g.pz.M <= 1024;  // several planes an SM
+    if (20LL * g.px.M <= 11 * sms && planes <= 5 * sms && !small) return std::min(n, kMaxBranches);
     return n == 3 ? 3 : 2;
 }
 struct Branches {
