@@ -655,7 +655,8 @@ cudaError_t enqueue_iteration(tdda_core* c, int first, int n, int slot, cudaStre
 //  - one for plane blocks that take nearly all of an SM's shared memory where the
 //    last wave is nearly full or the launch long, whose tails are short beside what
 //    the branches cost (41 x 90 x 23, three, 1.9 waves: 113 us, in three 116;
-//    96 x 96 x 24: six 449 us, in two 453; eight 600 and 605; twelve 870 and 898).
+//    96 x 96 x 24: six 449 us, in two 453; eight 600 and 605; twelve 870 and 898:
+//    the one plane size, 192 x 48, that this line was measured on).
 constexpr int kMaxBranches = 4;
 template <typename T> int solve_branches(const tdda_core* c, int n) {
     const Geom& g = c->g;
