@@ -377,11 +377,15 @@ typedef struct {
     int x_form, x_tile;  /* the chosen configuration (now set on the core) */
     int ncand;           /* candidates timed: 3, or 1 (form 1) where the x length has no register form */
     int form[4], tile[4];
-    double ms[4];        /* average ms of one FP32 A-product of nrhs right-hand sides, per candidate */
+    double ms[4];        /* average ms of half an FP32 step of nrhs right-hand sides (one product with its
+                          * vector updates), per candidate */
 } tdda_xpass_tune;
-/* Autotuner of the FP32 x pass: times `reps` plain FP32 A-products of nrhs
- * right-hand sides (CUDA events on the core's stream, after one warm-up) for
- * every candidate form and tile, and sets the fastest on the core. */
+/* Autotuner of the FP32 product: times FP32 solver steps of nrhs right-hand sides
+ * (at least `reps` products; CUDA events, after a warm-up) for every candidate form
+ * and tile, and sets the fastest on the core.  The steps run on models of a plane
+ * wave that the call makes and frees (their device memory is that of nrhs models of
+ * a refined solve); a core of one material, which takes no models, times plain
+ * products. */
 tdda_status tdda_core_autotune(tdda_core* core, int nrhs, int reps, tdda_xpass_tune* out);
 
 /* Batch schedule of the FP32 products of a batched solve (no counterpart in the
@@ -400,12 +404,9 @@ typedef struct {
     double ms[4];        /* average ms of half an FP32 step of nrhs right-hand sides (one product with its
                           * vector updates), per candidate */
 } tdda_batch_tune;
-/* Autotuner of the batch schedule: times FP32 solver steps of nrhs right-hand
- * sides (at least `reps` products; CUDA events, after a warm-up) for each
- * candidate group size, as a solve runs them (the whole batch in its parallel
- * branches), and sets the fastest on the core.  The steps run on models of a
- * plane wave that the call makes and frees (their device memory is that of nrhs
- * models of a refined solve). */
+/* Autotuner of the batch schedule: times each candidate group size as
+ * tdda_core_autotune does, on steps as a solve runs them (the whole batch in its
+ * parallel branches), and sets the fastest on the core. */
 tdda_status tdda_core_autotune_batch(tdda_core* core, int nrhs, int reps, tdda_batch_tune* out);
 
 #ifdef __cplusplus

@@ -49,7 +49,7 @@ def _core(box, n):
 @pytest.mark.parametrize("box,n,branches", BRANCHES)
 def test_batch_tuner_times_the_branches_of_a_solve(box, n, branches, loop, monkeypatch):
     """The candidates are timed on solver steps, the whole batch in its branches: by the kernels that
-    eight more steps of each launch (twelve steps against four where 24 and 8 products are asked for)."""
+    eight more steps of each launch, in two rounds (24 products asked for, and 8)."""
     monkeypatch.setenv("TDDA_DEVICE_LOOP", loop)
     core, _ = _core(box, n)
 
@@ -65,18 +65,44 @@ def test_batch_tuner_times_the_branches_of_a_solve(box, n, branches, loop, monke
     sets = [branches if g == 0 else -(-n // g) for g in groups]
     ends = 2  # the step end after every fourth step
     assert groups[0] == 0
-    assert many - few == 16 * core.pass_count(tdda.FP32_REFINE) * sum(sets) + ends * len(groups)
+    assert many - few == 2 * (16 * core.pass_count(tdda.FP32_REFINE) * sum(sets) + ends * len(groups))
     core.close()
 
 
 @pytest.mark.gpu
-def test_batch_tuner_of_a_core_of_one_material():
+@pytest.mark.parametrize("box,n,branches", [((20, 20, 10), 1, 1), ((48, 6, 6), 3, 3), ((20, 24, 20), 5, 4), ((97, 12, 9), 2, 2)])
+def test_x_tuner_times_solver_steps(box, n, branches):
+    """The gather's tiles and the forms likewise: tiles tie on plain products and not in a step."""
+    core, _ = _core(box, n)
+
+    def tune(reps):
+        before = tdda.kernel_launches()
+        t = core.autotune(nrhs=n, reps=reps)
+        best = min(t["candidates"], key=lambda k: k["ms"])
+        assert (t["x_form"], t["x_tile"]) == (best["form"], best["tile"]) and best["ms"] > 0
+        return tdda.kernel_launches() - before, [(k["form"], k["tile"]) for k in t["candidates"]]
+
+    tune(8)
+    (few, cands), (many, _) = tune(8), tune(24)
+    want = 0
+    for form, tile in cands:
+        core.set_xpass(form, tile)
+        x_first = core.pass_names(tdda.FP32_REFINE)[0] == "k_xfwd"  # the z-y-x passes take no branches
+        want += 2 * (16 * core.pass_count(tdda.FP32_REFINE) * (branches if x_first else 1) + 2)
+    assert many - few == want
+    core.close()
+
+
+@pytest.mark.gpu
+def test_tuners_of_a_core_of_one_material():
     """Such a core has no models; its products are timed."""
     if tdda.device_count() < 1:
         pytest.skip("no CUDA device")
     c = tdda.AProductCore(9, 8, 7, lattice.bulk(9, 8, 7), 10.0, 520.0, MAT[:1], max_rhs=2)
     t = c.autotune_batch(nrhs=2, reps=2)
     assert [k["group"] for k in t["candidates"]] == [0, 1] and all(k["ms"] > 0 for k in t["candidates"])
+    t = c.autotune(nrhs=2, reps=2)
+    assert all(k["ms"] > 0 for k in t["candidates"])
     c.close()
 
 

@@ -230,8 +230,8 @@ class AProductCore {
     }
     std::array<int, 3> grid() const { return grid_; }
     tdda_core* handle() const { return h_; }
-    // Not in the reference: times the FP32 x pass's forms and tiles on this core's
-    // A-product of nrhs right-hand sides and keeps the fastest (tdda_core_autotune).
+    // Not in the reference: times the forms and tiles of the FP32 product on solver steps
+    // of nrhs right-hand sides on this core and keeps the fastest (tdda_core_autotune).
     tdda_xpass_tune autotune(int nrhs = 1, int reps = 10) {
         tdda_xpass_tune t{};
         check(tdda_core_autotune(h_, nrhs, reps, &t), "autotune");

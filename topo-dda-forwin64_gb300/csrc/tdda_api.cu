@@ -2598,37 +2598,58 @@ struct TimedBatch {
 };
 
 // Half the device time in ms of one FP32 solver step of the models (its two
-// products with their vector updates), in the core's batch schedule: at least
-// `reps` products, as the difference of two runs, so that neither what a solve
-// does before and after its steps nor the graph's capture counts.  (Plain products
-// leave out the vectors, beside which no group's work grid stays in L2: 96 x 96 x 24,
-// eight right-hand sides, in one launch or by twos 249 and 248 us a product, but 602
-// and 687 us a step.)
+// products with their vector updates), with the core's x configuration and batch
+// schedule: at least `reps` products, as the difference of a long and a short run,
+// each the faster of two, so that neither what a solve does before and after its
+// steps nor the graph's capture counts.  (Plain products leave out the vectors.
+// The gather's tiles tie there and not in a step: 64 x 64 x 16, 8 and 16 lines 31.6
+// and 31.3 us a product, 36.5 and 35.4 us a step; 41 x 90 x 23 43.3 either way, 64.0
+// and 61.1.  And a group's work grid stays in L2 there: 96 x 96 x 24, eight
+// right-hand sides, in one launch or by twos 249 and 248 us a product, 602 and 687
+// us a step.)
 tdda_status time_steps(tdda_core* c, std::vector<tdda_model*>& ms, int reps, double* out) {
     const int n = (int)ms.size();
-    const int runs[3] = {kChunk, kChunk, kChunk + kChunk * ((reps - 1) / (2 * kChunk) + 1)};  // steps: warm-up, two timed
+    const int steps[2] = {kChunk, kChunk + kChunk * ((reps - 1) / (2 * kChunk) + 1)};
     cudaEvent_t ev[2] = {};
     for (cudaEvent_t& e : ev) TDDA_CK(cudaEventCreate(&e));
-    float t[3] = {};
-    int it[3] = {};
+    float t[2] = {1e30f, 1e30f};
+    int it[2] = {};
     tdda_status st = TDDA_OK;
-    for (int k = 0; k < 3 && st == TDDA_OK; k++) {
-        for (int i = 0; i < n; i++) c->hst[i] = fresh_state(0.0, runs[k], 0);
+    for (int k = -1; k < 4 && st == TDDA_OK; k++) {  // a short run to warm up, then short, long, short, long
+        const int w = k < 0 ? 0 : k & 1;
+        for (int i = 0; i < n; i++) c->hst[i] = fresh_state(0.0, steps[w], 0);
         cudaError_t e = cudaMemcpyAsync(c->st32, c->hst, sizeof(SolveState) * n, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(ev[0], c->stream);
-        if (e == cudaSuccess) st = krylov<float>(c, n, true, runs[k]);
+        if (e == cudaSuccess) st = krylov<float>(c, n, true, steps[w]);
         if (e == cudaSuccess) e = cudaEventRecord(ev[1], c->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&t[k], ev[0], ev[1]);
+        float dt = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&dt, ev[0], ev[1]);
         if (e != cudaSuccess && st == TDDA_OK) st = cuda_fail(e, "timed steps");
-        it[k] = c->hst[0].it;
+        if (k >= 0) t[w] = std::min(t[w], dt), it[w] = c->hst[0].it;
     }
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
     // a solve that ends by itself (converged to the last bit, or not finite) takes the same
-    // steps in every schedule
-    *out = it[2] > it[1] ? (t[2] - t[1]) / (2.0 * (it[2] - it[1])) : t[2] / (2.0 * std::max(1, it[2]));
+    // steps in every candidate
+    *out = it[1] > it[0] && t[1] > t[0] ? (t[1] - t[0]) / (2.0 * (it[1] - it[0])) : t[1] / (2.0 * std::max(1, it[1]));
     return st;
 }
+
+// The time of a candidate of the tuners: on solver steps, or on plain products
+// where the core takes no models (one material).
+struct Timed {
+    tdda_core* c;
+    int nrhs, reps;
+    TimedBatch b;
+    tdda_status create() { return c->nmat > 1 ? b.create(c, nrhs) : TDDA_OK; }
+    tdda_status run(double* ms) {
+        if (!b.ms.empty()) return time_steps(c, b.ms, reps, ms);
+        double ms5[5];
+        TDDA_TRY(profile_products(c, TDDA_FP32_REFINE, nrhs, reps, ms5));
+        *ms = ms5[0] + ms5[1] + ms5[2] + ms5[3] + ms5[4];
+        return TDDA_OK;
+    }
+};
 
 // A captured solve step holds its pass kernels and their Geom: a new FP32 x-pass
 // configuration drops the FP32 step graphs (captured again on next use).
@@ -2689,16 +2710,16 @@ tdda_status tdda_core_autotune(tdda_core* c, int nrhs, int reps, tdda_xpass_tune
     out->form[nc] = 1, out->tile[nc++] = 0;
     out->ncand = nc;
     const int form0 = c->g.x_form, tile0 = c->g.x_tile;
+    Timed timed{c, nrhs, reps, {}};
+    TDDA_TRY(timed.create());
     int best = -1;
     for (int k = 0; k < nc; k++) {
-        double ms5[5];
         tdda_status st = set_xpass(c, out->form[k], out->tile[k]);
-        if (st == TDDA_OK) st = profile_products(c, TDDA_FP32_REFINE, nrhs, reps, ms5);
+        if (st == TDDA_OK) st = timed.run(&out->ms[k]);
         if (st != TDDA_OK) {
             set_xpass(c, form0, tile0);
             return st;
         }
-        out->ms[k] = ms5[0] + ms5[1] + ms5[2] + ms5[3] + ms5[4];
         if (best < 0 || out->ms[k] < out->ms[best]) best = k;
     }
     out->x_form = out->form[best];
@@ -2729,18 +2750,12 @@ tdda_status tdda_core_autotune_batch(tdda_core* c, int nrhs, int reps, tdda_batc
         if (g < nrhs) out->groups[nc++] = g;
     out->ncand = nc;
     const int group0 = c->group;
-    const bool models = c->nmat > 1;  // a core of one material takes products only
-    TimedBatch b;
-    if (models) TDDA_TRY(b.create(c, nrhs));
+    Timed timed{c, nrhs, reps, {}};
+    TDDA_TRY(timed.create());
     int best = -1;
     for (int k = 0; k < nc; k++) {
         tdda_status st = set_batch_group(c, out->groups[k]);
-        if (st == TDDA_OK && models) st = time_steps(c, b.ms, reps, &out->ms[k]);
-        if (st == TDDA_OK && !models) {
-            double ms5[5];
-            st = profile_products(c, TDDA_FP32_REFINE, nrhs, reps, ms5);
-            if (st == TDDA_OK) out->ms[k] = ms5[0] + ms5[1] + ms5[2] + ms5[3] + ms5[4];
-        }
+        if (st == TDDA_OK) st = timed.run(&out->ms[k]);
         if (st != TDDA_OK) {
             set_batch_group(c, group0);
             return st;

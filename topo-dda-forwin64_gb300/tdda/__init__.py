@@ -309,7 +309,8 @@ class AProductCore:
         _check(load().tdda_core_set_xpass(self.h, int(form), int(tile)), "tdda_core_set_xpass")
 
     def autotune(self, nrhs: int = 1, reps: int = 10) -> dict:
-        """Time the FP32 x-pass candidates on this core's A-product and keep the fastest."""
+        """Time the candidates of the FP32 product on solver steps of this core and keep the fastest
+        (ms: half a step, one product with its vector updates)."""
         t = XpassTune()
         _check(load().tdda_core_autotune(self.h, int(nrhs), int(reps), ctypes.byref(t)), "tdda_core_autotune")
         return {"x_form": t.x_form, "x_tile": t.x_tile,
