@@ -384,8 +384,8 @@ typedef struct {
  * (at least `reps` products; CUDA events, after a warm-up) for every candidate form
  * and tile, and sets the fastest on the core.  The steps run on models of a plane
  * wave that the call makes and frees (their device memory is that of nrhs models of
- * a refined solve); a core of one material, which takes no models, times plain
- * products. */
+ * a refined solve); where there is no memory for them, and on a core of one material,
+ * which takes no models, plain products are timed. */
 tdda_status tdda_core_autotune(tdda_core* core, int nrhs, int reps, tdda_xpass_tune* out);
 
 /* Batch schedule of the FP32 products of a batched solve (no counterpart in the

@@ -2592,9 +2592,11 @@ struct TimedBatch {
         TDDA_CK(cudaMemcpyAsync(c->rhs32, h32.data(), sizeof(RhsVecs<float>) * n, cudaMemcpyHostToDevice, c->stream));
         return TDDA_OK;
     }
-    ~TimedBatch() {
+    void clear() {
         for (tdda_model* m : ms) tdda_model_destroy(m);
+        ms.clear();
     }
+    ~TimedBatch() { clear(); }
 };
 
 // Half the device time in ms of one FP32 solver step of the models (its two
@@ -2636,12 +2638,17 @@ tdda_status time_steps(tdda_core* c, std::vector<tdda_model*>& ms, int reps, dou
 }
 
 // The time of a candidate of the tuners: on solver steps, or on plain products
-// where the core takes no models (one material).
+// where there are no models to run (a core of one material, no memory for them).
 struct Timed {
     tdda_core* c;
     int nrhs, reps;
     TimedBatch b;
-    tdda_status create() { return c->nmat > 1 ? b.create(c, nrhs) : TDDA_OK; }
+    void create() {
+        if (c->nmat < 2 || b.create(c, nrhs) == TDDA_OK) return;
+        b.clear();
+        g_err.clear();
+        cudaGetLastError();
+    }
     tdda_status run(double* ms) {
         if (!b.ms.empty()) return time_steps(c, b.ms, reps, ms);
         double ms5[5];
@@ -2711,7 +2718,7 @@ tdda_status tdda_core_autotune(tdda_core* c, int nrhs, int reps, tdda_xpass_tune
     out->ncand = nc;
     const int form0 = c->g.x_form, tile0 = c->g.x_tile;
     Timed timed{c, nrhs, reps, {}};
-    TDDA_TRY(timed.create());
+    timed.create();
     int best = -1;
     for (int k = 0; k < nc; k++) {
         tdda_status st = set_xpass(c, out->form[k], out->tile[k]);
@@ -2751,7 +2758,7 @@ tdda_status tdda_core_autotune_batch(tdda_core* c, int nrhs, int reps, tdda_batc
     out->ncand = nc;
     const int group0 = c->group;
     Timed timed{c, nrhs, reps, {}};
-    TDDA_TRY(timed.create());
+    timed.create();
     int best = -1;
     for (int k = 0; k < nc; k++) {
         tdda_status st = set_batch_group(c, out->groups[k]);
